@@ -31,6 +31,12 @@ MAIN_ON_MIRROR = ORACLE_DIR / "_ref" / "main_on_mirror"  # the reference's main.
 # the build recipe's default location.  Only build() reads it.
 REFERENCE_TREE = Path(os.environ.get("VOCALSIM_REFERENCE", "/root/reference"))
 
+
+def have_reference() -> bool:
+    """The tree holds the sources (an empty folder does not count)."""
+    return any(REFERENCE_TREE.glob("**/TwoMassModel.h"))
+
+
 _orc = None
 _ref = None
 
@@ -39,7 +45,7 @@ def build(force: bool = False) -> None:
     """Compile the oracle (and the reference pieces when the tree is present)."""
     if force or not LIB.exists():
         subprocess.run(["make", "-s", "-C", str(ORACLE_DIR)], check=True)
-    if REFERENCE_TREE.exists() and (force or not (REF_LIB.exists() and REF_ENGINE.exists() and REF_ENGINE_G.exists())):
+    if have_reference() and (force or not (REF_LIB.exists() and REF_ENGINE.exists() and REF_ENGINE_G.exists())):
         subprocess.run(["make", "-s", "-C", str(ORACLE_DIR), "-f", "Makefile.ref",
                         f"REF={REFERENCE_TREE}", "all"], check=True)
 
@@ -48,7 +54,7 @@ def build_main_on_mirror(force: bool = False) -> None:
     """Compile the reference's own driver (src/main.cu, unchanged) against the
     library's C++ mirror headers; needs the reference tree and the built
     libvocalsim_b200.so."""
-    if REFERENCE_TREE.exists() and (force or not MAIN_ON_MIRROR.exists()):
+    if have_reference() and (force or not MAIN_ON_MIRROR.exists()):
         subprocess.run(["make", "-s", "-C", str(ORACLE_DIR), "-f", "Makefile.ref", f"REF={REFERENCE_TREE}",
                         "main_on_mirror"], check=True)
 
