@@ -125,6 +125,9 @@ struct vs_batch {
     int adj_rows = 0;                      // rows per strip of the strip forms (0 = the form's default)
     int adj_graph_rows = 0;
     ClusterConfig cluster{};
+    int npairs = 0;                        // fast_math: most distinct descriptor pairs of a tube
+    ResidentPlan resident;                 // the cluster shape's launch (no order: the kernels of `cluster`)
+    int* d_order = nullptr;                // ResidentPlan::order
     // adjoint: checkpoints of the last checkpointed forward, history, adjoint planes
     int64_t ck_steps = 0;                  // steps of the checkpointed forward (0 = none)
     int ck_every = 0;
@@ -172,6 +175,8 @@ struct vs_batch {
         if (d_tubes) cudaFree(d_tubes);
         if (d_tiles) cudaFree(d_tiles);
         if (d_rs) cudaFree(d_rs);
+        if (d_order) cudaFree(d_order);
+        d_order = nullptr;
         if (d_trace) cudaFree(d_trace);
         if (ckpt) cudaFree(ckpt);
         if (adj_mem) cudaFree(adj_mem);
@@ -293,6 +298,13 @@ bool cluster_fits(const vs_batch* b) {
     if (b->cluster_state == 0) {
         vs_batch* m = const_cast<vs_batch*>(b);
         m->cluster_state = -1;
+        bool any_tmm = false;
+        for (const TubeGrid& g : b->grids) any_tmm = any_tmm || g.tmm;
+        if (!b->wall && b->fast && !any_tmm &&
+            resident_plan(b->grids.data(), (int)b->grids.size(), b->npairs, &m->resident)) {
+            m->cluster_state = 1;
+            return true;
+        }
         if (b->grids.size() <= kMaxClusterTubes && !b->wall) {
             int H = 0, W = 0, pitch = 0, min_rows = INT32_MAX;
             bool tmm = false;
@@ -341,7 +353,7 @@ int default_shape(const vs_batch* b) {
     // are resident at once (measured, fast_math: 2 and 4 tubes 1.36 us per
     // step against 2.6 on the strips; past one wave of clusters the strips win)
     const int n = (int)b->grids.size();
-    if (shape_fits(b, cluster_shape()) && (n == 1 || (b->cluster.form != 0 && n <= b->cluster.nclusters)))
+    if (shape_fits(b, cluster_shape()) && (n == 1 || !b->resident.order.empty() || (b->cluster.form != 0 && n <= b->cluster.nclusters)))
         return cluster_shape();
     int64_t cells = 0;
     for (const TubeGrid& g : b->grids) cells += g.dims.interior_cells;
@@ -755,9 +767,26 @@ void upload_static_tube(vs_batch* b, size_t i) {
 // Every tube's read-only block (depth planes, codes, fast_math descriptors
 // and tables, from TubeDev::dP on, as laid out in the arena), staged on the
 // host in parallel and copied with one transfer per tube.
+// Distinct descriptors of two adjacent cells (even column first), the count
+// the resident kernel's tables are sized for.
+int descriptor_pairs(const TubeGrid& g, const std::vector<uint8_t>& desc) {
+    std::vector<uint64_t> seen(1024, 0);
+    for (int r = 0; r < g.H; ++r) {
+        const uint8_t* d = &desc[(size_t)r * g.pitch];
+        for (int c = 0; c < g.pitch; c += 2) {
+            const unsigned key = d[c] | (unsigned)d[c + 1] << 8;
+            seen[key >> 6] |= 1ull << (key & 63);
+        }
+    }
+    int n = 0;
+    for (uint64_t v : seen) n += __builtin_popcountll(v);
+    return n;
+}
+
 void upload_static(vs_batch* b) {
     const size_t n = b->grids.size();
     std::vector<std::vector<char>> img(n);
+    std::vector<int> pairs(n, 0);
     parallel_for(n, [&](size_t i) {
         const TubeGrid& g = b->grids[i];
         const TubeDev& t = b->h_tubes[i];
@@ -772,6 +801,7 @@ void upload_static(vs_batch* b) {
             std::vector<uint8_t> desc;
             std::vector<float> ta, tb;
             build_descriptors(g, desc, ta, tb, &b->h_tubes[i].ndesc, !b->fast);
+            pairs[i] = descriptor_pairs(g, desc);
             std::memcpy(m.data() + at(t.desc), desc.data(), desc.size());
             std::memcpy(m.data() + at(t.desc_a), ta.data(), ta.size() * sizeof(float));
             std::memcpy(m.data() + at(t.desc_b), tb.data(), tb.size() * sizeof(float));
@@ -791,11 +821,13 @@ void upload_static(vs_batch* b) {
             std::vector<uint8_t> desc;
             std::vector<float> ta, tb;
             build_descriptors(g, desc, ta, tb, &b->h_tubes[i].ndesc, !b->fast);
+            pairs[i] = descriptor_pairs(g, desc);
             std::memcpy(m.data() + at(t.desc), desc.data(), desc.size());
             std::memcpy(m.data() + at(t.desc_a), ta.data(), ta.size() * sizeof(float));
             std::memcpy(m.data() + at(t.desc_b), tb.data(), tb.size() * sizeof(float));
         }
     });
+    for (int k : pairs) b->npairs = std::max(b->npairs, k);
     for (size_t i = 0; i < n; ++i) {
         if (img[i].empty()) continue;
         const TubeDev& t = b->h_tubes[i];
@@ -920,6 +952,17 @@ void create_batch(int n, const vs_params* params, const vs_geometry* geoms, vs_b
     b->shape = default_shape(b);
 }
 
+// `count` steps of every tube on the resident kernel.
+void issue_resident(vs_batch* b, int64_t count, bool hist) {
+    const ResidentPlan& plan = b->resident;
+    if (!b->d_order) {
+        ck(cudaMalloc(&b->d_order, plan.order.size() * sizeof(int)), "cudaMalloc(tube order)");
+        ck(cudaMemcpy(b->d_order, plan.order.data(), plan.order.size() * sizeof(int), cudaMemcpyHostToDevice),
+           "upload tube order");
+    }
+    ck(launch_resident_run(b->d_tubes, b->d_rs, b->d_order, count, plan, b->stream, hist), "resident launch");
+}
+
 // Issue `count` steps from the device step counter (graph chunks of kChunk
 // plus direct launches), RunState already set with bsel = 0.  With a
 // two-step shape the launches alternate between the parity set and the third
@@ -927,6 +970,10 @@ void create_batch(int n, const vs_params* params, const vs_geometry* geoms, vs_b
 // count ends with one launch of the batch's single-step shape, so the state
 // of the final step is in its parity set (bsel = 0) when the call returns.
 void issue_steps(vs_batch* b, int64_t count) {
+    if (tile_shape(b->shape).kind == SHAPE_CLUSTER && !b->resident.order.empty()) {
+        issue_resident(b, count, false);
+        return;
+    }
     if (tile_shape(b->shape).kind == SHAPE_CLUSTER) {
         ck(launch_cluster_run(b->d_tubes, b->d_rs, count, b->fast, b->cluster, b->stream, (int)b->grids.size()),
            "cluster launch");
@@ -1205,7 +1252,8 @@ void run_adjoint(vs_batch* b, const float* gtrace, float* gdP, float* gdX, float
     // each segment with one cluster launch that stores every step's state;
     // otherwise, with fast_math, a full segment (K even) is recomputed two
     // steps per launch by the two-step kernel, which needs the third state set
-    const bool hist_cluster = n == 1 && tile_shape(b->shape).kind == SHAPE_CLUSTER && b->cluster.form != 0;
+    const bool hist_cluster =
+        tile_shape(b->shape).kind == SHAPE_CLUSTER && (!b->resident.order.empty() || (n == 1 && b->cluster.form != 0));
     const bool hist_two = !hist_cluster && b->fast && K % 2 == 0;
     if (hist_two) ensure_third_set(b);
     // device memory per tube, all zeroed per call: history (K+1 slots x 3
@@ -1378,7 +1426,10 @@ void run_adjoint(vs_batch* b, const float* gtrace, float* gdP, float* gdX, float
         ck(cudaEventRecord(ev[3 * k], b->stream), "event");
         ck(launch_history_seed(b->d_tubes, n, max_plane, (int)(start & 1), b->stream), "history seed");
         if (hist_cluster) {
-            ck(launch_cluster_run(b->d_tubes, b->d_rs, len, b->fast, b->cluster, b->stream), "history (cluster)");
+            if (!b->resident.order.empty())
+                issue_resident(b, len, true);
+            else
+                ck(launch_cluster_run(b->d_tubes, b->d_rs, len, b->fast, b->cluster, b->stream), "history (cluster)");
             ck(cudaEventRecord(ev[3 * k + 1], b->stream), "event");
             if (len == K) ck(cudaGraphLaunch(b->adj_graph, b->stream), "reverse graph");
             else

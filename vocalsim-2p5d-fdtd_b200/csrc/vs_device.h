@@ -4,6 +4,7 @@
 
 #include <cstdint>
 #include <string>
+#include <vector>
 
 #include <cuda_runtime_api.h>
 
@@ -217,6 +218,21 @@ bool cluster_config(int H, int W, int pitch, bool fast, bool tmm, ClusterConfig*
 // (bsel = 0) and stay there.
 cudaError_t launch_cluster_run(const TubeDev* tube, RunState* rs, int64_t steps, bool fast, const ClusterConfig& c,
                                cudaStream_t stream, int ntubes = 1);
+
+// Launch plan of the resident kernel (vs_resident.cu) for a batch of
+// table-source tubes in the reciprocal form.
+struct ResidentPlan {
+    int ctas = 0, threads = 0, smem = 0;      // per tube: cluster size; CTA threads and shared memory
+    std::vector<int> order;                   // tubes in launch order (empty: no plan)
+};
+// false when some tube does not fit; npairs = the most distinct descriptors of
+// two adjacent cells of a tube.
+bool resident_plan(const TubeGrid* grids, int n, int npairs, ResidentPlan* out);
+// `steps` steps of every tube from RunState::step, which then advances (order:
+// the plan's in device memory); `hist` also stores every step's state into the
+// tubes' history.
+cudaError_t launch_resident_run(const TubeDev* tubes, RunState* rs, const int* order, int64_t steps,
+                                const ResidentPlan& plan, cudaStream_t stream, bool hist);
 
 // Launch one time step (local index `local` after RunState::step) of every
 // strip or band in `tiles` with the compiled shape `shape`; `wall` selects
