@@ -39,7 +39,7 @@ def run(case, fast, shape):
     return out, [b.fields(i) for i in (0, len(tubes) - 1)]
 
 
-@pytest.mark.parametrize("fast", [1])
+@pytest.mark.parametrize("fast", [1, 0])
 @pytest.mark.parametrize("case", CASES)
 def test_resident_equals_the_step_kernels(case, fast, cuda_ok):
     a, fa = run(case, fast, CLUSTER)
@@ -51,7 +51,7 @@ def test_resident_equals_the_step_kernels(case, fast, cuda_ok):
             np.testing.assert_array_equal(u, v)
 
 
-@pytest.mark.parametrize("fast", [1])
+@pytest.mark.parametrize("fast", [1, 0])
 def test_resident_history_gives_the_step_kernels_gradients(fast, cuda_ok):
     """The adjoint's recomputation on the resident kernel: the same states, so the same gradients."""
     tubes = [S.batch_tube(k)[:2] for k in range(3)]

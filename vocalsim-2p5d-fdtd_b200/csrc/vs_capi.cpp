@@ -125,7 +125,7 @@ struct vs_batch {
     int adj_rows = 0;                      // rows per strip of the strip forms (0 = the form's default)
     int adj_graph_rows = 0;
     ClusterConfig cluster{};
-    int npairs = 0;                        // fast_math: most distinct descriptor pairs of a tube
+    int npairs = 0;                        // most distinct descriptors of two adjacent cells of a tube
     ResidentPlan resident;                 // the cluster shape's launch (no order: the kernels of `cluster`)
     int* d_order = nullptr;                // ResidentPlan::order
     // adjoint: checkpoints of the last checkpointed forward, history, adjoint planes
@@ -298,10 +298,11 @@ bool cluster_fits(const vs_batch* b) {
     if (b->cluster_state == 0) {
         vs_batch* m = const_cast<vs_batch*>(b);
         m->cluster_state = -1;
-        bool any_tmm = false;
-        for (const TubeGrid& g : b->grids) any_tmm = any_tmm || g.tmm;
-        if (!b->wall && b->fast && !any_tmm &&
-            resident_plan(b->grids.data(), (int)b->grids.size(), b->npairs, &m->resident)) {
+        // the resident kernel: table sources, every tube's neighbourhoods in its tables
+        bool plain = !b->wall && b->desc;
+        for (const TubeGrid& g : b->grids) plain = plain && !g.tmm;
+        for (const TubeDev& t : b->h_tubes) plain = plain && t.ndesc > 0;
+        if (plain && resident_plan(b->grids.data(), (int)b->grids.size(), b->npairs, b->fast, &m->resident)) {
             m->cluster_state = 1;
             return true;
         }

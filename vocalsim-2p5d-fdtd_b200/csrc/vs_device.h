@@ -220,14 +220,15 @@ cudaError_t launch_cluster_run(const TubeDev* tube, RunState* rs, int64_t steps,
                                cudaStream_t stream, int ntubes = 1);
 
 // Launch plan of the resident kernel (vs_resident.cu) for a batch of
-// table-source tubes in the reciprocal form.
+// table-source tubes.
 struct ResidentPlan {
     int ctas = 0, threads = 0, smem = 0;      // per tube: cluster size; CTA threads and shared memory
+    bool fast = true;                         // reciprocal form, else the reference arithmetic
     std::vector<int> order;                   // tubes in launch order (empty: no plan)
 };
 // false when some tube does not fit; npairs = the most distinct descriptors of
 // two adjacent cells of a tube.
-bool resident_plan(const TubeGrid* grids, int n, int npairs, ResidentPlan* out);
+bool resident_plan(const TubeGrid* grids, int n, int npairs, bool fast, ResidentPlan* out);
 // `steps` steps of every tube from RunState::step, which then advances (order:
 // the plan's in device memory); `hist` also stores every step's state into the
 // tubes' history.

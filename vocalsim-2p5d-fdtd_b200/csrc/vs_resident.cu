@@ -172,8 +172,9 @@ constexpr int kMaxRows = 12;      // rows per lane the registers hold (72 of 128
 // the row above it) at a constant stride: rcp(dP) and dX, dY, descriptors.
 constexpr int kGhostBytes = 2 * 512 + 2 * 256;
 constexpr int kGhostB = 2 * 512;
-constexpr int kRecBytes = 512 + 256 + 64;
-constexpr int kRecY = 512, kRecD = 768;
+constexpr int kRecY = 512, kRecP = 768;         // (rcp(dP), dX) at 0, dY, and in the reference arithmetic dP
+__host__ __device__ constexpr int rec_desc(bool exact) { return exact ? 1024 : 768; }
+__host__ __device__ constexpr int rec_bytes(bool exact) { return rec_desc(exact) + 64; }
 // per (group, tile edge): Vx dX to the left of it (row i at i - 1), then P' to the right of it
 // (rows 2 .. R-1 at i - 2, rows 1 and R at kMaxRows and kMaxRows + 1)
 constexpr int kEdgeP = kMaxRows;
@@ -182,21 +183,24 @@ constexpr int kEdgeFloats = 2 * kMaxRows + 4;
 constexpr int kHashSlots = 1024;
 constexpr int kMaxPairs = 128;                   // descriptor pairs of a tube (vowel tubes: 50 to 75)
 constexpr int kTab = kMaxPairs * 16;             // one table of 16-byte entries
-// fixed offsets: barriers, give-up flags, (-1, -1); then the pair tables: (g, ce), (al_x, al_y),
-// (zo_x, -zi_x), (zo_y, -zi_y)
-constexpr int kOffBar = 0, kOffFail = 16, kOffM1 = 32, kOffTab = 64, kOffGhost = kOffTab + 4 * kTab;
+// fixed offsets: barriers, give-up flags, (-1, -1); then the pair tables.  Reciprocal form: (g, ce),
+// (al_x, al_y), (zo_x, -zi_x), (zo_y, -zi_y).  Reference arithmetic: (-sP, -), (-den_x, 1 / den_x),
+// (-den_y, 1 / den_y), (mB_x, -mS_x), (A_x, B_x), (mB_y, -mS_y), (A_y, B_y), (W_x, W_y); the wall term's
+// pressure is A Pc + B Pn.
+constexpr int kOffBar = 0, kOffFail = 16, kOffM1 = 32, kOffTab = 64;
+__host__ __device__ constexpr int off_ghost(bool exact) { return kOffTab + (exact ? 8 : 4) * kTab; }
 
 struct ResLayout {
     int edge, rec, bytes;
 };
 
-__host__ __device__ inline ResLayout res_layout(int nwx, int ng, int nrow) {
+__host__ __device__ inline ResLayout res_layout(int nwx, int ng, int nrow, bool exact) {
     ResLayout L{};
     const int ghost = (ng + 1) * nwx * kGhostBytes;
     // the ghost rows' place also holds the pair table's hash while the block starts
-    L.edge = kOffGhost + (ghost > kHashSlots * 4 ? ghost : kHashSlots * 4);
+    L.edge = off_ghost(exact) + (ghost > kHashSlots * 4 ? ghost : kHashSlots * 4);
     L.rec = L.edge + (ng * (nwx + 1) * kEdgeFloats * 4 + 15) / 16 * 16;
-    L.bytes = (L.rec + nwx * (nrow + 2) * kRecBytes + 127) / 128 * 128;
+    L.bytes = (L.rec + nwx * (nrow + 2) * rec_bytes(exact) + 127) / 128 * 128;
     return L;
 }
 
@@ -215,12 +219,43 @@ struct TileCtx {
     int tube;
 };
 
+// a[k] / b[k] for N pairs, correctly rounded: nb = -b, y = 1 / b correctly
+// rounded (0 where the result is 0 by definition: ring and no-pressure cells).
+// Two fused corrections of a y (P. Markstein, IBM J. Res. Dev. 34(1), 1990) give
+// the IEEE quotient while nothing on the way leaves the normal range; a warp
+// that meets a numerator outside 2^-80 .. 2^100 (the first steps of a wave
+// front) divides the block again with the IEEE division.
+template <int N>
+__device__ __forceinline__ void quotients(u64 (&a)[N], const u64 (&nb)[N], const u64 (&y)[N]) {
+    u64 q[N], r[N];
+    bool odd = false;
+    float top = 0.0f;
+    auto tiny = [](float v) { return (__float_as_uint(v) & 0x7fffffffu) - 1u < 0x17800000u - 1u; };   // 0 < |v| < 2^-80
+    static_for<0, N>([&](auto kc) {
+        odd = odd || tiny(plo(a[kc])) || tiny(phi(a[kc]));
+        top = fmaxf(top, fmaxf(fabsf(plo(a[kc])), fabsf(phi(a[kc]))));
+    });
+    static_for<0, N>([&](auto kc) { q[kc] = mul2(a[kc], y[kc]); });
+    static_for<0, N>([&](auto kc) { r[kc] = fma2(nb[kc], q[kc], a[kc]); });
+    static_for<0, N>([&](auto kc) { q[kc] = fma2(r[kc], y[kc], q[kc]); });
+    static_for<0, N>([&](auto kc) { r[kc] = fma2(nb[kc], q[kc], a[kc]); });
+    static_for<0, N>([&](auto kc) { q[kc] = fma2(r[kc], y[kc], q[kc]); });
+    if (__any_sync(0xffffffffu, odd || top > 1.2676506e30f)) {
+        auto div = [](float v, float nd, float rc) { return rc == 0.0f ? 0.0f : fdiv_z(v, -nd); };
+        static_for<0, N>([&](auto kc) {
+            q[kc] = pk(div(plo(a[kc]), plo(nb[kc]), plo(y[kc])), div(phi(a[kc]), phi(nb[kc]), phi(y[kc])));
+        });
+    }
+    static_for<0, N>([&](auto kc) { a[kc] = q[kc]; });
+}
+
 // Up to kRegRows rows per group the maps and the pressure and velocity factors
 // stay in registers too; taller groups read them from shared memory.
 constexpr int kRegRows = 3;
 
-template <int R, bool HIST>
+template <int R, bool HIST, bool EXACT>
 __device__ __forceinline__ void run_tile(const TileCtx& X) {
+    constexpr int kOffGhost = off_ghost(EXACT), kRecBytes = rec_bytes(EXACT), kRecD = rec_desc(EXACT);
     constexpr unsigned kAll = 0xffffffffu;
     constexpr bool inReg = R <= kRegRows;
     const TubeDev* __restrict__ T = X.T;
@@ -256,6 +291,8 @@ __device__ __forceinline__ void run_tile(const TileCtx& X) {
     auto zx_at = [&](uint32_t o) { return lds128(o + kOffTab + 2 * kTab); };
     auto zy_at = [&](uint32_t o) { return lds128(o + kOffTab + 3 * kTab); };
     auto ce_at = [&](uint32_t o) { return lds64(o + kOffTab + 8); };
+    auto tab_at = [&](uint32_t o, int k) { return lds128(o + kOffTab + k * kTab); };
+    auto dp_s = [&](int i) { return lds64(recY + (kRecP - kRecY) + i * kRecBytes); };
     const uint32_t first = lane == 0 ? ~0u : 0u, last = lane == 31 ? ~0u : 0u;
 
     // ---- state of the group's rows (0 = the row above, whose P is kept too)
@@ -263,6 +300,7 @@ __device__ __forceinline__ void run_tile(const TileCtx& X) {
     u64 rX[inReg ? R + 1 : 1], rY[inReg ? R + 2 : 1], rP[inReg ? R + 1 : 1];
     u64 rG[inReg ? R + 1 : 1], rAx[inReg ? R + 1 : 1], rAy[inReg ? R + 1 : 1];
     uint32_t gnm = 0;                        // per row: the tile has a cell with wall or source terms
+    uint32_t dvm = 0;                        // reference arithmetic, per row: a velocity division
     bool srcm = false;
     {
         const float* __restrict__ gP = T->P[0] + par0 * pl;
@@ -276,17 +314,31 @@ __device__ __forceinline__ void run_tile(const TileCtx& X) {
             if constexpr (inReg) { rP[i] = m.x; rX[i] = m.y; rY[i] = dy_s(i); }
             const unsigned d = id_at(i);
             const u64 gg = g_at(d);
-            const ulonglong2 al = al_at(d);
-            const float4 zx = ldsf4(d + kOffTab + 2 * kTab), zy = ldsf4(d + kOffTab + 3 * kTab);
-            const u64 ce2 = ce_at(d);
-            const float2 ce = make_float2(plo(ce2), phi(ce2));
-            if constexpr (inReg) { rG[i] = gg; rAx[i] = al.x; rAy[i] = al.y; }
-            const bool c = ce.x != 0.0f || ce.y != 0.0f;
-            const bool gn = c || zx.x != 0.0f || zx.y != 0.0f || zx.z != 0.0f || zx.w != 0.0f || zy.x != 0.0f ||
-                            zy.y != 0.0f || zy.z != 0.0f || zy.w != 0.0f;
-            if (i > 0) {
-                gnm |= (uint32_t)__any_sync(kAll, gn) << i;
-                srcm = srcm || __any_sync(kAll, c);
+            if constexpr (EXACT) {
+                const ulonglong2 bx = tab_at(d, 4), by = tab_at(d, 6), mx = tab_at(d, 3), my = tab_at(d, 5);
+                const ulonglong2 w = tab_at(d, 7), qx = tab_at(d, 1), qy = tab_at(d, 2);
+                const u64 one = pk(1.0f, 1.0f);
+                if constexpr (inReg) { rG[i] = gg; rAx[i] = dp_s(i); }
+                const bool c = w.x != 0 || w.y != 0;
+                const bool gn = c || bx.x != 0 || bx.y != 0 || by.x != 0 || by.y != 0 || mx.x != one || my.x != one;
+                if (i > 0) {
+                    gnm |= (uint32_t)__any_sync(kAll, gn) << i;
+                    dvm |= (uint32_t)__any_sync(kAll, gn || qx.y != one || qy.y != one) << i;
+                    srcm = srcm || __any_sync(kAll, c);
+                }
+            } else {
+                const ulonglong2 al = al_at(d);
+                const float4 zx = ldsf4(d + kOffTab + 2 * kTab), zy = ldsf4(d + kOffTab + 3 * kTab);
+                const u64 ce2 = ce_at(d);
+                const float2 ce = make_float2(plo(ce2), phi(ce2));
+                if constexpr (inReg) { rG[i] = gg; rAx[i] = al.x; rAy[i] = al.y; }
+                const bool c = ce.x != 0.0f || ce.y != 0.0f;
+                const bool gn = c || zx.x != 0.0f || zx.y != 0.0f || zx.z != 0.0f || zx.w != 0.0f || zy.x != 0.0f ||
+                                zy.y != 0.0f || zy.z != 0.0f || zy.w != 0.0f;
+                if (i > 0) {
+                    gnm |= (uint32_t)__any_sync(kAll, gn) << i;
+                    srcm = srcm || __any_sync(kAll, c);
+                }
             }
             asm volatile("" ::: "memory");
         });
@@ -301,7 +353,9 @@ __device__ __forceinline__ void run_tile(const TileCtx& X) {
         else return dy_s(decltype(ic)::value);
     };
     const float K1 = T->K1, bco = T->bcoef;
-    const u64 nK1 = pk(-K1, -K1);
+    const u64 cK = EXACT ? pk(K1, K1) : pk(-K1, -K1);
+    const bool eigen = (T->flags & TUBE_EIGEN) != 0;
+    const u64 zz = pk(T->zinv, T->zinv);
     const u64 m1 = lds64(sb + kOffM1);
     const u64 bc = pk(in0 ? bco : 0.0f, in1 ? bco : 0.0f);        // ring columns keep zero velocities
     const float* __restrict__ src = T->src + n0;
@@ -367,7 +421,23 @@ __device__ __forceinline__ void run_tile(const TileCtx& X) {
                     u[k] = pk(fsub(plo(u[k]), ul[k]), fsub(phi(u[k]), plo(u[k])));
                 });
                 static_for<0, N>([&](auto kc) { sum[kc] = add2(u[kc], sum[kc]); });
-                static_for<0, N>([&](auto kc) { sum[kc] = mul2(nK1, sum[kc]); });
+                static_for<0, N>([&](auto kc) { sum[kc] = mul2(cK, sum[kc]); });
+                if constexpr (EXACT) {
+                    // (P dP - K1 S) / ((1 + sigma) dP), or / (sigma dP + dP); -sP in gf
+                    u64 dp[N];
+                    static_for<0, N>([&](auto kc) {
+                        constexpr int k = decltype(kc)::value, i = row[k];
+                        if constexpr (inReg) dp[k] = rAx[i];
+                        else dp[k] = dp_s(i);
+                    });
+                    static_for<0, N>([&](auto kc) { gf[kc] = mul2(gf[kc], dp[kc]); });
+                    if (eigen) static_for<0, N>([&](auto kc) { gf[kc] = diff2(gf[kc], dp[kc], m1); });
+                    static_for<0, N>([&](auto kc) { dp[kc] = mul2(P[row[kc]], dp[kc]); });
+                    static_for<0, N>([&](auto kc) { sum[kc] = diff2(dp[kc], sum[kc], m1); });
+                    quotients<N>(sum, gf, rp);
+                    static_for<0, N>([&](auto kc) { P[row[kc]] = sum[kc]; });
+                    return;
+                }
                 static_for<0, N>([&](auto kc) { P[row[kc]] = fma2(sum[kc], rp[kc], P[row[kc]]); });
                 static_for<0, N>([&](auto kc) { P[row[kc]] = mul2(P[row[kc]], gf[kc]); });
             };
@@ -447,7 +517,7 @@ __device__ __forceinline__ void run_tile(const TileCtx& X) {
                     if constexpr (!inReg) d[kc] = id_at(row[kc]);
                 });
                 static_for<0, N>([&](auto kc) { prx[kc] = __shfl_down_sync(kAll, plo(P[row[kc]]), 1); });
-                static_for<0, N>([&](auto kc) {
+                if constexpr (!EXACT) static_for<0, N>([&](auto kc) {
                     constexpr int k = decltype(kc)::value, i = row[k];
                     if constexpr (inReg) {
                         ax[k] = rAx[i];
@@ -468,6 +538,48 @@ __device__ __forceinline__ void run_tile(const TileCtx& X) {
                 static_for<0, N>([&](auto kc) { dx[kc] = mul2(bc, dx[kc]); });
                 static_for<0, N>([&](auto kc) { VY[row[kc]] = diff2(VY[row[kc]], dy[kc], m1); });
                 static_for<0, N>([&](auto kc) { VX[row[kc]] = diff2(VX[row[kc]], dx[kc], m1); });
+                if constexpr (EXACT) {
+                    if (!(dvm & mask)) return;
+                    if constexpr (inReg) static_for<0, N>([&](auto kc) { d[kc] = id_at(row[kc]); });
+                    if (gnm & mask) {
+                        // mB V - ..., the source's and the wall's terms, in the reference's order
+                        static_for<0, N>([&](auto kc) {
+                            constexpr int k = decltype(kc)::value, i = row[k];
+                            const ulonglong2 mx = tab_at(d[k], 3), my = tab_at(d[k], 5);
+                            VX[i] = mul2(VX[i], mx.x);
+                            VY[i] = mul2(VY[i], my.x);
+                            if (srcm) {
+                                const ulonglong2 w = tab_at(d[k], 7);
+                                const u64 ee = pk(exe, exe);
+                                VX[i] = diff2(VX[i], mul2(mul2(ee, w.x), mx.y), m1);
+                                VY[i] = diff2(VY[i], mul2(mul2(ee, w.y), my.y), m1);
+                            }
+                            const ulonglong2 bx = tab_at(d[k], 4), by = tab_at(d[k], 6);
+                            const u64 px = fma2(bx.x, P[i], mul2(bx.y, pk(phi(P[i]), prx[k])));
+                            const u64 py = fma2(by.x, P[i], mul2(by.y, P[i - 1]));
+                            VX[i] = diff2(VX[i], mul2(mx.y, mul2(px, zz)), m1);
+                            VY[i] = diff2(VY[i], mul2(my.y, mul2(py, zz)), m1);
+                        });
+                    }
+                    u64 num[N], nden[N], rec1[N];
+                    static_for<0, N>([&](auto kc) {
+                        const ulonglong2 v = tab_at(d[kc], 1);
+                        num[kc] = VX[row[kc]];
+                        nden[kc] = v.x;
+                        rec1[kc] = v.y;
+                    });
+                    quotients<N>(num, nden, rec1);
+                    static_for<0, N>([&](auto kc) {
+                        const ulonglong2 v = tab_at(d[kc], 2);
+                        VX[row[kc]] = num[kc];
+                        num[kc] = VY[row[kc]];
+                        nden[kc] = v.x;
+                        rec1[kc] = v.y;
+                    });
+                    quotients<N>(num, nden, rec1);
+                    static_for<0, N>([&](auto kc) { VY[row[kc]] = num[kc]; });
+                    return;
+                }
                 static_for<0, N>([&](auto kc) { VY[row[kc]] = mul2(VY[row[kc]], ay[kc]); });
                 static_for<0, N>([&](auto kc) { VX[row[kc]] = mul2(VX[row[kc]], ax[kc]); });
                 if (gnm & mask) {
@@ -566,11 +678,11 @@ __device__ __forceinline__ void run_tile(const TileCtx& X) {
 }
 
 // The step loop of the warp's group height.
-template <int R, bool HIST>
+template <int R, bool HIST, bool EXACT>
 __device__ __forceinline__ void run_rows(int rows, const TileCtx& X) {
     if constexpr (R <= kMaxRows) {
-        if (rows == R) run_tile<R, HIST>(X);
-        else run_rows<R + 1, HIST>(rows, X);
+        if (rows == R) run_tile<R, HIST, EXACT>(X);
+        else run_rows<R + 1, HIST, EXACT>(rows, X);
     }
 }
 
@@ -584,11 +696,12 @@ __device__ __forceinline__ void run_idle(const TileCtx& X) {
     }
 }
 
-template <bool HIST>
+template <bool HIST, bool EXACT>
 __global__ void __launch_bounds__(kMaxWarps * 32, 1)
 resident_kernel(const TubeDev* __restrict__ tubes, RunState* __restrict__ rs,
                 const int* __restrict__ order, int nsteps) {
     extern __shared__ __align__(128) unsigned char res_smem[];
+    constexpr int kOffGhost = off_ghost(EXACT), kRecBytes = rec_bytes(EXACT), kRecD = rec_desc(EXACT);
     cg::cluster_group cluster = cg::this_cluster();
     TileCtx X;
     X.C = (int)cluster.num_blocks();
@@ -608,7 +721,7 @@ resident_kernel(const TubeDev* __restrict__ tubes, RunState* __restrict__ rs,
     X.nwx = (W - 2) / kTileCols + 1;                 // columns 0 .. W-2
     X.ng = nw / X.nwx;
     X.nwy = min(X.ng, nrow);
-    X.L = res_layout(X.nwx, X.ng, nrow);
+    X.L = res_layout(X.nwx, X.ng, nrow, EXACT);
     const int lanes = X.nwx * 32;
 
     // ---- maps, descriptors and tables into shared memory; ghost rows of the first step
@@ -628,7 +741,7 @@ resident_kernel(const TubeDev* __restrict__ tubes, RunState* __restrict__ rs,
             const int j = e / lanes, l = e - j * lanes;
             const int r = ra - 1 + j, x = 2 * l;
             const bool row_in = r >= 1 && r <= H - 2;
-            float rc[2] = {0.0f, 0.0f}, dx[2] = {0.0f, 0.0f}, dy[2] = {0.0f, 0.0f};
+            float rc[2] = {0.0f, 0.0f}, dp[2] = {0.0f, 0.0f}, dx[2] = {0.0f, 0.0f}, dy[2] = {0.0f, 0.0f};
             uint32_t d = 0;
             for (int h = 0; h < 2; ++h) {
                 const int c = x + h;
@@ -637,13 +750,22 @@ resident_kernel(const TubeDev* __restrict__ tubes, RunState* __restrict__ rs,
                 dx[h] = dP[pl + o];
                 dy[h] = dP[2 * pl + o];
                 if (row_in && c >= 1 && c <= W - 2) {
-                    rc[h] = rcp_approx(dP[o]);
-                    d |= (uint32_t)T->desc[o] << (8 * h);
+                    const uint32_t id = T->desc[o];
+                    d |= id << (8 * h);
+                    dp[h] = dP[o];
+                    if constexpr (EXACT) {
+                        const float4 a = T->desc_a[id];
+                        if (!(__float_as_uint(a.w) & EXD_PZERO))
+                            rc[h] = fdiv(1.0f, pressure_den(a.x, dp[h], (T->flags & TUBE_EIGEN) != 0));
+                    } else {
+                        rc[h] = rcp_approx(dp[h]);
+                    }
                 }
             }
             unsigned char* row = res_smem + X.L.rec + ((l >> 5) * (nrow + 2) + j) * kRecBytes;
             *reinterpret_cast<float4*>(row + (l & 31) * 16) = make_float4(rc[0], rc[1], dx[0], dx[1]);
             *reinterpret_cast<float2*>(row + kRecY + (l & 31) * 8) = make_float2(dy[0], dy[1]);
+            if constexpr (EXACT) *reinterpret_cast<float2*>(row + kRecP + (l & 31) * 8) = make_float2(dp[0], dp[1]);
             *reinterpret_cast<uint16_t*>(row + kRecD + (l & 31) * 2) = (uint16_t)d;
             // the descriptor pair into the hash table (at most kMaxPairs distinct ones)
             uint32_t s = start(d);
@@ -664,6 +786,26 @@ resident_kernel(const TubeDev* __restrict__ tubes, RunState* __restrict__ rs,
             const float4 a0 = T->desc_a[d & 0xff], a1 = T->desc_a[d >> 8];
             const float4 b0 = T->desc_b[d & 0xff], b1 = T->desc_b[d >> 8];
             float4* tab = reinterpret_cast<float4*>(res_smem + kOffTab) + id;
+            if constexpr (EXACT) {
+                const uint32_t f0 = __float_as_uint(a0.w), f1 = __float_as_uint(a1.w);
+                const bool z = T->zinv != 0.0f;
+                auto mb = [](uint32_t f) { return (f & EXD_MB) ? 1.0f : 0.0f; };
+                auto wa = [z](uint32_t f) {
+                    return z && (f & EXD_WALL) && (f & EXD_WALL_PC) ? ((f & EXD_NOUT1) ? 1.0f : 0.707106f) : 0.0f;
+                };
+                auto wb = [z](uint32_t f) { return z && (f & EXD_WALL) && !(f & EXD_WALL_PC) ? -1.0f : 0.0f; };
+                const uint32_t g0 = f0 >> EXD_Y_SHIFT, g1 = f1 >> EXD_Y_SHIFT;
+                tab[0] = make_float4(-a0.x, -a1.x, 0.0f, 0.0f);
+                tab[kMaxPairs] = make_float4(-a0.y, -a1.y, fdiv(1.0f, a0.y), fdiv(1.0f, a1.y));
+                tab[2 * kMaxPairs] = make_float4(-a0.z, -a1.z, fdiv(1.0f, a0.z), fdiv(1.0f, a1.z));
+                tab[3 * kMaxPairs] = make_float4(mb(f0), mb(f1), -b0.x, -b1.x);
+                tab[4 * kMaxPairs] = make_float4(wa(f0), wa(f1), wb(f0), wb(f1));
+                tab[5 * kMaxPairs] = make_float4(mb(g0), mb(g1), -b0.z, -b1.z);
+                tab[6 * kMaxPairs] = make_float4(wa(g0), wa(g1), wb(g0), wb(g1));
+                tab[7 * kMaxPairs] = make_float4((f0 & EXD_SRC) ? b0.y : 0.0f, (f1 & EXD_SRC) ? b1.y : 0.0f,
+                                                 (g0 & EXD_SRC) ? b0.w : 0.0f, (g1 & EXD_SRC) ? b1.w : 0.0f);
+                continue;
+            }
             tab[0] = make_float4(a0.z, a1.z, a0.w, a1.w);
             tab[kMaxPairs] = make_float4(a0.x, a1.x, a0.y, a1.y);
             tab[2 * kMaxPairs] = make_float4(b0.x, b1.x, -b0.y, -b1.y);
@@ -734,7 +876,7 @@ resident_kernel(const TubeDev* __restrict__ tubes, RunState* __restrict__ rs,
         const int a = (int)(((int64_t)X.g * nrow) / X.nwy), b = (int)(((int64_t)(X.g + 1) * nrow) / X.nwy);
         X.j0 = a;
         X.r0 = ra + a;
-        run_rows<1, HIST>(b - a, X);
+        run_rows<1, HIST, EXACT>(b - a, X);
     } else {
         run_idle(X);
     }
@@ -762,15 +904,17 @@ void cluster_launch(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr, const Re
 
 }  // namespace
 
-bool resident_plan(const TubeGrid* grids, int n, int npairs, ResidentPlan* out) {
+bool resident_plan(const TubeGrid* grids, int n, int npairs, bool fast, ResidentPlan* out) {
     *out = ResidentPlan{};
+    const void* plain = fast ? (const void*)resident_kernel<false, false> : (const void*)resident_kernel<false, true>;
+    const void* hist = fast ? (const void*)resident_kernel<true, false> : (const void*)resident_kernel<true, true>;
     if (npairs < 1 || npairs > kMaxPairs) return false;
     int dev = 0, optin = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess)
         return false;
-    for (const void* fn : {(const void*)resident_kernel<false>, (const void*)resident_kernel<true>})
+    for (const void* fn : {plain, hist})
         if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, optin) != cudaSuccess ||
             cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
             cudaGetLastError();
@@ -790,6 +934,7 @@ bool resident_plan(const TubeGrid* grids, int n, int npairs, ResidentPlan* out) 
     for (int C : {1, 2, 3, 4, 6, 8, 12, 16}) {
         ResidentPlan p;
         p.ctas = C;
+        p.fast = fast;
         bool ok = true;
         for (int i = 0; i < n && ok; ++i) {
             const int NR = grids[i].H - 2, nwx = (grids[i].W - 2) / kTileCols + 1;
@@ -797,12 +942,12 @@ bool resident_plan(const TubeGrid* grids, int n, int npairs, ResidentPlan* out) 
             const int nrow = (NR + C - 1) / C, ng = std::min(kMaxWarps / nwx, nrow), R = (nrow + ng - 1) / ng;
             p.threads = std::max(p.threads, 32 * ng * nwx);
             ok = R <= kMaxRows;
-            t[(size_t)i] = 0.5 + 0.013 * R * ng * nwx;
+            t[(size_t)i] = 0.5 + (fast ? 0.013 : 0.02) * R * ng * nwx;
         }
         if (!ok) continue;
         for (int i = 0; i < n; ++i) {
             const int NR = grids[i].H - 2, nwx = (grids[i].W - 2) / kTileCols + 1;
-            p.smem = std::max(p.smem, res_layout(nwx, p.threads / 32 / nwx, (NR + C - 1) / C).bytes);
+            p.smem = std::max(p.smem, res_layout(nwx, p.threads / 32 / nwx, (NR + C - 1) / C, !fast).bytes);
             idx[(size_t)i] = i;
         }
         if (p.smem > optin) continue;
@@ -830,10 +975,12 @@ bool resident_plan(const TubeGrid* grids, int n, int npairs, ResidentPlan* out) 
     cudaLaunchAttribute attr[1];
     cluster_launch(&cfg, attr, *out);
     int resident = 0;
-    if (cudaOccupancyMaxActiveClusters(&resident, (const void*)resident_kernel<true>, &cfg) != cudaSuccess ||
+    if (cudaOccupancyMaxActiveClusters(&resident, hist, &cfg) != cudaSuccess ||
         resident < 1) {
         cudaGetLastError();
         *out = ResidentPlan{};
+    const void* plain = fast ? (const void*)resident_kernel<false, false> : (const void*)resident_kernel<false, true>;
+    const void* hist = fast ? (const void*)resident_kernel<true, false> : (const void*)resident_kernel<true, true>;
         return false;
     }
     return true;
@@ -848,7 +995,9 @@ cudaError_t launch_resident_run(const TubeDev* tubes, RunState* rs, const int* o
     cudaError_t e = cudaSuccess;
     while (steps > 0 && e == cudaSuccess) {
         const int k = (int)std::min<int64_t>(steps, 1 << 30);
-        e = cudaLaunchKernelEx(&cfg, hist ? resident_kernel<true> : resident_kernel<false>, tubes, rs, order, k);
+        const auto fn = plan.fast ? (hist ? resident_kernel<true, false> : resident_kernel<false, false>)
+                                  : (hist ? resident_kernel<true, true> : resident_kernel<false, true>);
+        e = cudaLaunchKernelEx(&cfg, fn, tubes, rs, order, k);
         // the step counter advances after every cluster has run: a cluster
         // that starts later reads RunState::step then
         if (e == cudaSuccess) e = launch_advance(rs, k, stream);
