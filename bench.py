@@ -485,13 +485,20 @@ def run_b200(args, rank, world):
     value = job_cells * sim_steps / (ms_step / 1e3) / 1e9
     # a two-step shape advances two time steps per launch and moves the state
     # planes once per launch: algorithmic bytes per launch = 37 B x cells
+    # (the resident kernel runs all steps in one launch and moves the planes and
+    # maps once; a launch that advances the step counter follows it)
     per_launch = V.tile_shape_steps(tile)
+    whole = per_launch == 0
+    if whole:
+        per_launch = sim_steps
     step_launches = sim_steps // per_launch + sim_steps % per_launch
-    launches_per_forward = step_launches + math.ceil(sim_steps / 128)
+    launches_per_forward = 2 if whole else step_launches + math.ceil(sim_steps / 128)
     launch_ms = ms_step / step_launches        # average per step-kernel launch incl. graph gaps
     # algorithmic bytes per launch = 37 B per cell-update x the cell-updates one
     # launch performs (cells x time steps per launch)
-    achieved_gbs = BYTES_PER_CELL_UPDATE * cells * per_launch / (launch_ms / 1e3) / 1e9
+    launch_bytes = (BYTES_PER_CELL_UPDATE * cells + 4 * len(ps) * sim_steps if whole
+                    else BYTES_PER_CELL_UPDATE * cells * per_launch)
+    achieved_gbs = launch_bytes / (launch_ms / 1e3) / 1e9
     peak, peak_kind = hbm_peak()
     prof = profiled_kernel(cells, tile, fast)
 
@@ -634,7 +641,7 @@ def run_b200(args, rank, world):
                                 if args.strong else f"tube sharding x{world} (no collective)"),
                 "arithmetic": "reciprocal form (fast_math=1)" if fast else "reference rounding (fast_math=0)",
                 "l2": "state + maps per GPU > 126 MB L2 and 33075 launches per timed step; no flush"},
-        "roofline": {"bound": "hbm", "achieved": round(achieved_gbs, 1), "peak": peak, "unit": "GB/s",
+        "roofline": {"bound": "on-chip latency" if whole else "hbm", "achieved": round(achieved_gbs, 1), "peak": peak, "unit": "GB/s",
                      "frac": round(achieved_gbs / peak, 4), "traffic": prof["traffic"],
                      # DRAM bytes the launch really moves (ncu, same kernel and workload) per
                      # launch time: the two-step kernel moves the planes once per two steps
@@ -645,8 +652,10 @@ def run_b200(args, rank, world):
                      # roofline (37 B per cell-update moved once per step at the peak)
                      "gcell_roofline": round(peak / BYTES_PER_CELL_UPDATE, 1),
                      "gcell_frac": round(value / world / (peak / BYTES_PER_CELL_UPDATE), 4),
-                     "note": f"{BYTES_PER_CELL_UPDATE} B algorithmic per cell-update x {cells} cells x {per_launch} "
-                             f"time step(s) per launch / mean launch time {launch_ms * 1e3:.2f} us; peak {peak_kind}; "
+                     "note": (f"{launch_bytes} B per launch (planes and maps once, traces) / " if whole else
+                              f"{BYTES_PER_CELL_UPDATE} B algorithmic per cell-update x {cells} cells x {per_launch} "
+                              f"time step(s) per launch / ") +
+                             f"mean launch time {launch_ms * 1e3:.2f} us; peak {peak_kind}; "
                              f"dram_frac and issue_active_pct from the committed ncu summary of the same kernel"},
         "gpu_launches": args.steps * launches_per_forward,
         "clocks": clocks.summary(),

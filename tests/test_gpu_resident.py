@@ -1,4 +1,4 @@
-"""The resident kernel (vs_resident.cu, the cluster shape of table-source batches): a whole run of
+"""The resident kernel (vs_resident.cu, the cluster shape): a whole run of
 every tube on its own cluster, against the step kernels, value for value."""
 import numpy as np
 import pytest
@@ -24,6 +24,10 @@ CASES = {
     "sine_mouth": ((201,), [S.vowel_tube(k) for k in range(3)],
                    dict(cross_sectional_shape=2, source_type=0, mouth_radiation_cond=1)),
     "eigen_2d": ((150,), [S.vowel_tube(5)], dict(cross_sectional_shape=2, engine=2, fdtd_solver_type=0)),
+    "voiced": ((1, 120, 33), [S.vowel_tube(k) for k in range(2)],
+               dict(cross_sectional_shape=2, source_type=2, tmm_ps_pa=800.0)),
+    "voiced_f64": ((2, 201), [S.vowel_tube(3)],
+                   dict(cross_sectional_shape=2, source_type=2, tmm_ps_pa=800.0, tmm_f64=1)),
     "many": ((33, 40), [S.batch_tube(k)[:2] for k in range(90)], dict(cross_sectional_shape=2)),
     "fine": ((64,), [S.batch_tube(k)[:2] for k in range(2)], dict(cross_sectional_shape=2, srate_mul=30)),
 }
@@ -51,15 +55,16 @@ def test_resident_equals_the_step_kernels(case, fast, cuda_ok):
             np.testing.assert_array_equal(u, v)
 
 
+@pytest.mark.parametrize("kw", [{}, dict(source_type=2, tmm_ps_pa=800.0, tmm_f64=1)])
 @pytest.mark.parametrize("fast", [1, 0])
-def test_resident_history_gives_the_step_kernels_gradients(fast, cuda_ok):
+def test_resident_history_gives_the_step_kernels_gradients(fast, kw, cuda_ok):
     """The adjoint's recomputation on the resident kernel: the same states, so the same gradients."""
     tubes = [S.batch_tube(k)[:2] for k in range(3)]
     rng = np.random.default_rng(5)
     seed = rng.standard_normal((3, 300)).astype(np.float32)
     res = []
     for shape in (CLUSTER, 21 if fast else 7):
-        b = V.Batch([V.params(cross_sectional_shape=2, fast_math=fast) for _ in tubes],
+        b = V.Batch([V.params(cross_sectional_shape=2, fast_math=fast, **kw) for _ in tubes],
                     [V.Geometry(*t) for t in tubes])
         b.set_tile(shape)
         tr = b.forward_ckpt(300, 128)

@@ -12,6 +12,7 @@ import os
 import shutil
 import subprocess
 import sys
+from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
 PKG = Path(__file__).resolve().parent
@@ -24,7 +25,8 @@ ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "--fmad=false", "-Xcompiler", "-fPIC,-ffp-contract=off,-O2",
               f"-I{INCLUDE}", "-Wno-deprecated-gpu-targets"]
 
-SOURCES = ["vs_grid.cpp", "vs_capi.cpp", "vs_step.cu", "vs_cluster.cu", "vs_resident.cu", "vs_noalloc.cu", "vs_adjoint.cu", "vs_mapbuild.cu", "vs_spectrum.cu",
+SOURCES = ["vs_grid.cpp", "vs_capi.cpp", "vs_step.cu", "vs_cluster.cu", "vs_resident.cu", "vs_resident_fast.cu", "vs_resident_exact.cu",
+           "vs_resident_fast_tmm.cu", "vs_resident_exact_tmm.cu", "vs_noalloc.cu", "vs_adjoint.cu", "vs_mapbuild.cu", "vs_spectrum.cu",
            "vs_sections.cu", "vs_audio.cu", "vs_shapes.cpp"]
 
 
@@ -46,7 +48,7 @@ def build(force: bool = False, verbose: bool = False) -> Path:
     OBJ.mkdir(exist_ok=True)
     LIB.parent.mkdir(exist_ok=True)
     headers = list(CSRC.glob("*.h")) + list(CSRC.glob("*.cuh")) + [INCLUDE / "vocalsim_b200.h"]
-    objs = []
+    objs, jobs = [], []
     for src in SOURCES:
         s = CSRC / src
         o = OBJ / (s.stem + ".o")
@@ -56,7 +58,9 @@ def build(force: bool = False, verbose: bool = False) -> Path:
             cmd = [nvcc(), *NVCC_FLAGS, *ARCH, *lang, "-c", str(s), "-o", str(o)]
             if verbose:
                 print(" ".join(cmd))
-            subprocess.run(cmd, check=True)
+            jobs.append(cmd)
+    with ThreadPoolExecutor(max_workers=os.cpu_count() or 1) as pool:
+        list(pool.map(lambda cmd: subprocess.run(cmd, check=True), jobs))
     if force or _stale(LIB, objs):
         # cuFFT (vs_formants) is linked dynamically from the toolkit next to nvcc
         cuda_lib = Path(nvcc()).resolve().parent.parent / "lib64"

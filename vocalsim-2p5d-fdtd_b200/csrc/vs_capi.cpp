@@ -298,9 +298,8 @@ bool cluster_fits(const vs_batch* b) {
     if (b->cluster_state == 0) {
         vs_batch* m = const_cast<vs_batch*>(b);
         m->cluster_state = -1;
-        // the resident kernel: table sources, every tube's neighbourhoods in its tables
+        // the resident kernel: every tube's neighbourhoods in its tables
         bool plain = !b->wall && b->desc;
-        for (const TubeGrid& g : b->grids) plain = plain && !g.tmm;
         for (const TubeDev& t : b->h_tubes) plain = plain && t.ndesc > 0;
         if (plain && resident_plan(b->grids.data(), (int)b->grids.size(), b->npairs, b->fast, &m->resident)) {
             m->cluster_state = 1;

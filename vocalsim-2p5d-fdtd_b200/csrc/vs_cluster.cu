@@ -361,31 +361,6 @@ cluster_kernel(const TubeDev* __restrict__ Tp, RunState* __restrict__ rs, int64_
 //                a CTA may still read it.  Waits are bounded; a CTA that gives
 //                up reports VS_ERR_TIMEOUT, and every CTA meets at a final
 //                cluster barrier before any exits.
-// The two-mass model's state and its prepared step, kept in shared memory by
-// the one thread that runs it, so that the model's registers do not count
-// against every thread's budget (the helpers are not inlined).
-struct TmmSlot {
-    TmmState64 s64;
-    TmmPrep64 prep64;
-    TmmState s32;
-    TmmPrep prep32;
-};
-
-__device__ __noinline__ void tmm_slot_prepare(const TubeDev* __restrict__ T, TmmSlot* slot, bool tmm64) {
-    if (tmm64) slot->prep64 = tmm_prepare64(T->tmmd, T->tmmx, slot->s64);
-    else slot->prep32 = tmm_prepare(T->tmmc, slot->s32);
-}
-
-__device__ __noinline__ float tmm_slot_finish(TmmSlot* slot, bool tmm64, float p1) {
-    return tmm64 ? tmm_finish64(slot->prep64, slot->s64, p1) : tmm_finish(slot->prep32, slot->s32, p1);
-}
-
-// The model's current state as the adjoint's two-mass history keeps it.
-__device__ __noinline__ void tmm_slot_hist(const TmmSlot* slot, bool tmm64, double* h) {
-    if (tmm64) tmm_to_hist(slot->s64, h);
-    else tmm_to_hist(slot->s32, h);
-}
-
 struct RegLayout {
     int pitch, nw, rmax;
     size_t gT, gVyB, dX0, eUX, eP, tab, sig, exe, tmm, bar, exr, bytes;   // byte offsets

@@ -219,13 +219,19 @@ bool cluster_config(int H, int W, int pitch, bool fast, bool tmm, ClusterConfig*
 cudaError_t launch_cluster_run(const TubeDev* tube, RunState* rs, int64_t steps, bool fast, const ClusterConfig& c,
                                cudaStream_t stream, int ntubes = 1);
 
-// Launch plan of the resident kernel (vs_resident.cu) for a batch of
-// table-source tubes.
+// Launch plan of the resident kernel (vs_resident.cu) for a batch.
 struct ResidentPlan {
-    int ctas = 0, threads = 0, smem = 0;      // per tube: cluster size; CTA threads and shared memory
+    int ctas = 0, warps = 0, threads = 0, smem = 0;   // cluster size; per CTA: tile warps, threads, shared memory
     bool fast = true;                         // reciprocal form, else the reference arithmetic
+    bool tmm = false;                         // some tube has the two-mass source
     std::vector<int> order;                   // tubes in launch order (empty: no plan)
 };
+// The kernel's variants, plain or storing the history.
+using ResidentFn = void (*)(const TubeDev*, RunState*, const int*, int, int);
+ResidentFn resident_fast(bool hist);
+ResidentFn resident_exact(bool hist);
+ResidentFn resident_fast_tmm(bool hist);
+ResidentFn resident_exact_tmm(bool hist);
 // false when some tube does not fit; npairs = the most distinct descriptors of
 // two adjacent cells of a tube.
 bool resident_plan(const TubeGrid* grids, int n, int npairs, bool fast, ResidentPlan* out);
