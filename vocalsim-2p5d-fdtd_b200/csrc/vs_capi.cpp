@@ -307,15 +307,13 @@ bool cluster_fits(const vs_batch* b) {
         }
         if (b->grids.size() <= kMaxClusterTubes && !b->wall) {
             int H = 0, W = 0, pitch = 0, min_rows = INT32_MAX;
-            bool tmm = false;
             for (const TubeGrid& g : b->grids) {
                 H = std::max(H, g.H);
                 W = std::max(W, g.W);
                 pitch = std::max(pitch, g.pitch);
                 min_rows = std::min(min_rows, g.H - 2);
-                tmm = tmm || g.tmm;
             }
-            if (cluster_config(H, W, pitch, b->fast, tmm, &m->cluster) && m->cluster.ctas <= min_rows)
+            if (cluster_config(H, W, pitch, b->fast, &m->cluster) && m->cluster.ctas <= min_rows)
                 m->cluster_state = 1;
         }
     }
@@ -348,13 +346,11 @@ int single_step_shape(const vs_batch* b) {
 }
 
 int default_shape(const vs_batch* b) {
-    // a single tube keeps its state on one thread-block cluster for the whole
-    // run, and so does every tube of a batch whose clusters (register form)
-    // are resident at once (measured, fast_math: 2 and 4 tubes 1.36 us per
-    // step against 2.6 on the strips; past one wave of clusters the strips win)
-    const int n = (int)b->grids.size();
-    if (shape_fits(b, cluster_shape()) && (n == 1 || !b->resident.order.empty() || (b->cluster.form != 0 && n <= b->cluster.nclusters)))
-        return cluster_shape();
+    // the resident kernel wherever the tubes fit it: it is the fastest from one
+    // tube to 256 (us per step against the two-step strips: 5 tubes 0.74 / 2.7,
+    // 96 tubes 4.0 / 7.6, 256 tubes 8.4 / 17.4); a single tube that does not
+    // fit still keeps its state on one cluster
+    if (shape_fits(b, cluster_shape()) && (!b->resident.order.empty() || b->grids.size() == 1)) return cluster_shape();
     int64_t cells = 0;
     for (const TubeGrid& g : b->grids) cells += g.dims.interior_cells;
     const int two = two_step_shape(cells);
@@ -1248,12 +1244,12 @@ void run_adjoint(vs_batch* b, const float* gtrace, float* gdP, float* gdX, float
     if (form == ADJ_FORM_AUTO) form = (!any_tmm && strips8 >= 4 * (int64_t)sms) ? ADJ_FORM_STRIPS2 : ADJ_FORM_TILES;
     if (form == ADJ_FORM_STRIPS2 && any_tmm) form = ADJ_FORM_STRIPS;
     const int rows = b->adj_rows ? b->adj_rows : (form == ADJ_FORM_STRIPS2 ? 8 : 4);
-    // a single tube that steps on the cluster kernel (register form) recomputes
-    // each segment with one cluster launch that stores every step's state;
-    // otherwise, with fast_math, a full segment (K even) is recomputed two
-    // steps per launch by the two-step kernel, which needs the third state set
+    // a batch on the resident kernel recomputes each segment with one launch
+    // that stores every step's state; otherwise, with fast_math, a full segment
+    // (K even) is recomputed two steps per launch by the two-step kernel, which
+    // needs the third state set
     const bool hist_cluster =
-        tile_shape(b->shape).kind == SHAPE_CLUSTER && (!b->resident.order.empty() || (n == 1 && b->cluster.form != 0));
+        tile_shape(b->shape).kind == SHAPE_CLUSTER && !b->resident.order.empty();
     const bool hist_two = !hist_cluster && b->fast && K % 2 == 0;
     if (hist_two) ensure_third_set(b);
     // device memory per tube, all zeroed per call: history (K+1 slots x 3
@@ -1426,10 +1422,7 @@ void run_adjoint(vs_batch* b, const float* gtrace, float* gdP, float* gdX, float
         ck(cudaEventRecord(ev[3 * k], b->stream), "event");
         ck(launch_history_seed(b->d_tubes, n, max_plane, (int)(start & 1), b->stream), "history seed");
         if (hist_cluster) {
-            if (!b->resident.order.empty())
-                issue_resident(b, len, true);
-            else
-                ck(launch_cluster_run(b->d_tubes, b->d_rs, len, b->fast, b->cluster, b->stream), "history (cluster)");
+            issue_resident(b, len, true);
             ck(cudaEventRecord(ev[3 * k + 1], b->stream), "event");
             if (len == K) ck(cudaGraphLaunch(b->adj_graph, b->stream), "reverse graph");
             else

@@ -255,31 +255,6 @@ __device__ __forceinline__ void tmm_to_hist(const S& s, double* h) {
     h[3] = s.x2_curr; h[4] = s.ug_old; h[5] = s.ug_curr;
 }
 
-// The two-mass model's state and its prepared step, kept in shared memory by
-// the one thread that runs it, so that the model's registers do not count
-// against every thread's budget (the helpers are not inlined).
-struct TmmSlot {
-    TmmState64 s64;
-    TmmPrep64 prep64;
-    TmmState s32;
-    TmmPrep prep32;
-};
-
-__device__ __noinline__ void tmm_slot_prepare(const TubeDev* __restrict__ T, TmmSlot* slot, bool tmm64) {
-    if (tmm64) slot->prep64 = tmm_prepare64(T->tmmd, T->tmmx, slot->s64);
-    else slot->prep32 = tmm_prepare(T->tmmc, slot->s32);
-}
-
-__device__ __noinline__ float tmm_slot_finish(TmmSlot* slot, bool tmm64, float p1) {
-    return tmm64 ? tmm_finish64(slot->prep64, slot->s64, p1) : tmm_finish(slot->prep32, slot->s32, p1);
-}
-
-// The model's current state as the adjoint's two-mass history keeps it.
-__device__ __noinline__ void tmm_slot_hist(const TmmSlot* slot, bool tmm64, double* h) {
-    if (tmm64) tmm_to_hist(slot->s64, h);
-    else tmm_to_hist(slot->s32, h);
-}
-
 // Two-mass steps n and n+1 for the two-step kernels: the state of step n is
 // in the parity slot (from_x = false) or the third slot, that of step n+2
 // goes to the other one (stored by the owning strip only, which also writes

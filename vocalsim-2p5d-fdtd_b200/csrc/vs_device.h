@@ -194,23 +194,15 @@ TileShape tile_shape(int i);
 // thread-block cluster, every step of a run in one launch (vs_cluster.cu).
 int cluster_shape();
 
-// Launch configuration of the cluster kernel for one tube.
+// Launch configuration of the shared-memory cluster kernel for one tube.
 struct ClusterConfig {
     int ctas = 0, threads = 0, rows_max = 0;
-    int cols = 0;         // column threads (threads less the two-mass warp of form 2)
     size_t smem = 0;
-    int form = 0;         // 0: band in shared memory; 1: register-resident columns (rows_max <= rmax),
-                          // cluster barrier per step; 2: the same, neighbour-to-neighbour exchange;
-                          // 3: form 2 with the two-mass model in an extra warp
-    int rmax = 0;
-    int nclusters = 0;    // clusters of this configuration resident on the device at once
 };
 // Cluster size (16, 8 or 4 CTAs), threads and shared memory for a tube of
 // H x W cells (row pitch `pitch`) on the current device, or false when none
-// fits; sets the kernel attributes it needs.  `tmm`: the tube has the
-// two-mass source (its excitation value reaches every CTA each step, which
-// the cluster barrier form does faster than the neighbour exchange).
-bool cluster_config(int H, int W, int pitch, bool fast, bool tmm, ClusterConfig* out);
+// fits; sets the kernel attributes it needs.
+bool cluster_config(int H, int W, int pitch, bool fast, ClusterConfig* out);
 // `steps` time steps of the `ntubes` tubes from `tube` on (device), one
 // thread-block cluster per tube (configuration c, sized for the largest of
 // them), from RunState::step, in one launch; then RunState::step advances by

@@ -77,19 +77,4 @@ __device__ __forceinline__ uint32_t cluster_addr(const void* local, int rank) {
     return r;
 }
 
-// Asynchronous stores into a cluster CTA's shared memory whose bytes count
-// against that CTA's mbarrier `bar` (both cluster addresses): the receiver
-// learns of their arrival from the mbarrier phase, the sender issues no fence.
-__device__ __forceinline__ void st_async_v2(uint32_t addr, float a, float b, uint32_t bar) {
-    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.b32 [%0], {%1, %2}, [%3];" ::"r"(addr),
-                 "r"(__float_as_uint(a)), "r"(__float_as_uint(b)), "r"(bar)
-                 : "memory");
-}
-
-__device__ __forceinline__ void st_async_b32(uint32_t addr, float a, uint32_t bar) {
-    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(addr),
-                 "r"(__float_as_uint(a)), "r"(bar)
-                 : "memory");
-}
-
 }  // namespace vsb

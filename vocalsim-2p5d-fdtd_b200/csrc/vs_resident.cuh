@@ -26,21 +26,28 @@
 //     receiver's mbarrier (double-buffered by step parity)
 //   CTA barrier; the next step's first and last group wait (bounded) for the
 //     neighbour CTAs' rows
-// Arithmetic: the reciprocal form (fast_math) of the other kernels, operation
-// for operation (rcp(dP) is formed once instead of every step), so the values
-// are theirs.  Neighbourhood factors (walls, PML, source) come from tables
-// indexed by the descriptors of the lane's two cells: a tube has some 50 to 75
-// distinct pairs, packed as the operations take them.  The wall and source
-// terms run only in blocks of rows that hold such a cell.  Cells outside the
-// frame and ring cells have zero coefficients and so keep their zeros.
+// Arithmetic: that of the other kernels, operation for operation, so the
+// values are theirs.  fast_math: the reciprocal form (rcp(dP) is formed once
+// instead of every step).  Reference arithmetic: the IEEE quotients from the
+// correctly rounded reciprocals, see quotients().  Neighbourhood factors (walls,
+// PML, source) come from tables indexed by the descriptors of the lane's two
+// cells: a tube has some 50 to 75 distinct pairs, packed as the operations take
+// them.  The wall and source terms run only in blocks of rows that hold such a
+// cell.  Cells outside the frame and ring cells have zero coefficients and so
+// keep their zeros.  The two-mass source runs in a warp of its own
+// (run_two_mass), one step ahead of the velocities it enters.
 //
-// What bounds it: no DRAM traffic in the loop; about 65 instructions per
-// 64-cell row and step at 0.4 per scheduler and cycle, half of the shared-memory
-// pipe, the rest the latency of a warp's own chain and the two barriers.
-// Scalar instead of packed operations (82 instructions) ran at the same time;
-// 64 registers for twice the warps spilled and were slower (16 us per step of
-// the 256-tube batch); 24 rows of state per SM in fewer, taller groups or tubes
-// of each size with their own cluster size were no faster (10.2-11.5 us).
+// What bounds it: no DRAM traffic in the loop.  256 vowel tubes in the
+// reciprocal form (2 CTAs of 16 warps a tube, 6 to 12 rows a lane): 8.4 us per
+// time step (two-step strips 17.4), about 65 instructions per 64-cell row and
+// step at 0.4 per scheduler and cycle, half of the shared-memory pipe, the rest
+// the latency of a warp's own chain and the two barriers.  One 55 x 253 tube
+// (16 CTAs, 1 or 2 rows a lane): 0.65 us per step, 1.5 in the reference
+// arithmetic (a band per CTA with cells in branches: 1.35 and 3.7); with the
+// double two-mass model 0.91 (1.70).  Measured and not kept: scalar instead of
+// packed operations (82 instructions, the same time); 64 registers for twice
+// the warps (spills, 16 us per step of the 256 tubes); 168 registers with 12
+// warps, taller groups, or a cluster size per tube (10.2 to 11.5 us).
 #pragma once
 
 #include <cooperative_groups.h>
@@ -109,6 +116,12 @@ __device__ __forceinline__ void group_sync(int id, int count) {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory");
 }
 
+constexpr int kStepBar = 15;                     // named barrier of the tile warps; the groups use 1 .. 8
+
+__device__ __forceinline__ void step_sync(int count) {
+    asm volatile("bar.sync %0, %1;" ::"n"(kStepBar), "r"(count) : "memory");
+}
+
 // A value and its step in one 8-byte word (single-copy atomic): written by one
 // thread, polled (bounded) by the readers.
 __device__ __forceinline__ u64 tagged(int n, float v) { return ((u64)(uint32_t)n << 32) | __float_as_uint(v); }
@@ -120,6 +133,9 @@ __device__ __forceinline__ bool poll_tagged(const volatile u64* w, int n, uint32
     return (uint32_t)(x >> 32) == (uint32_t)n;
 }
 
+// Asynchronous store into a cluster CTA's shared memory whose bytes count
+// against that CTA's mbarrier `bar` (both cluster addresses): the receiver
+// learns of its arrival from the mbarrier phase, the sender issues no fence.
 __device__ __forceinline__ void st_async_pair(uint32_t addr, u64 v, uint32_t bar) {
     asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(addr), "l"(v),
                  "r"(bar)
@@ -201,7 +217,6 @@ constexpr int kOffBar = 0, kOffFail = 16, kOffM1 = 32;
 // cell's P' by step parity
 constexpr int kExeRing = 32;
 constexpr int kOffRing = 64, kOffWord = kOffRing + 8 * kExeRing, kOffTab = kOffWord + 16;
-constexpr int kStepBar = 15;                     // named barrier of the tile warps; the groups use 1 .. 8
 __host__ __device__ constexpr int off_ghost(bool exact) { return kOffTab + (exact ? 8 : 4) * kTab; }
 
 struct ResLayout {
@@ -687,7 +702,7 @@ __device__ __forceinline__ void run_tile(const TileCtx& X) {
             }
             hist += 3 * pl;
         }
-        group_sync(kStepBar, 32 * X.nw);
+        step_sync(32 * X.nw);
         // a wait that ran out in this step: every warp sees it after this barrier
         if (sfail[p]) {
             for (int i = 0; i < 64; ++i) __nanosleep(1000);     // stores in flight land before the CTAs meet
@@ -723,7 +738,7 @@ __device__ __forceinline__ void run_idle(const TileCtx& X) {
     volatile int* sfail = reinterpret_cast<volatile int*>(X.sm + kOffFail);
     const int par0 = (int)(X.rs->step & 1);
     for (int m = 0; m < X.nsteps; ++m) {
-        group_sync(kStepBar, 32 * X.nw);
+        step_sync(32 * X.nw);
         if (sfail[(par0 + m) & 1]) break;
     }
 }
