@@ -1295,9 +1295,11 @@ void run_adjoint(vs_batch* b, const float* gtrace, float* gdP, float* gdX, float
     std::vector<std::vector<uint8_t>> adesc(n);
     std::vector<std::vector<float>> atab(n);
     size_t exc_total = 0;
-    for (int i = 0; i < n; ++i) {
+    parallel_for((size_t)n, [&](size_t i) {
         excitation_list(b->grids[i], b->h_tubes[i].plane, eoff[i], ecoef[i]);
         adjoint_coefficients(b->grids[i], adesc[i], atab[i]);
+    });
+    for (int i = 0; i < n; ++i) {
         exc_total += align_up(eoff[i].size() * sizeof(int32_t)) + align_up(ecoef[i].size() * sizeof(float)) +
                      align_up(adesc[i].size()) + align_up(atab[i].size() * sizeof(float));
     }
@@ -1439,6 +1441,7 @@ void run_adjoint(vs_batch* b, const float* gtrace, float* gdP, float* gdX, float
         ck(cudaEventRecord(ev[3 * k + 2], b->stream), "event");
         q ^= launches(len) & 1;
     }
+    ck(launch_gradients_out(b->d_tubes, b->d_adj, n, max_plane, b->stream), "gradients out");
     ck(cudaStreamSynchronize(b->stream), "adjoint sync");
     b->adj_recompute_ms = 0.0f;
     b->adj_reverse_ms = 0.0f;
@@ -1450,25 +1453,27 @@ void run_adjoint(vs_batch* b, const float* gtrace, float* gdP, float* gdX, float
         b->adj_reverse_ms += r;
     }
     for (cudaEvent_t e : ev) cudaEventDestroy(e);
-    // gradients to the caller, frame by frame (unpadded)
+    // gradients to the caller, frame by frame (unpadded floats, converted on the device)
     size_t cell_off = 0;
     for (int i = 0; i < n; ++i) {
         const TubeGrid& g = b->grids[i];
-        const size_t pe = (size_t)b->h_tubes[i].plane;
-        std::vector<double> host(4 * pe);
-        ck(cudaMemcpy(host.data(), adj[i].gP, 4 * pe * sizeof(double), cudaMemcpyDeviceToHost), "read gradients");
-        double z = 0.0;
-        for (int r = 0; r < g.H; ++r)
-            for (int c = 0; c < g.W; ++c) {
-                const size_t src = (size_t)r * g.pitch + c, dst = cell_off + (size_t)r * g.W + c;
-                if (gdP) gdP[dst] = (float)host[src];
-                if (gdX) gdX[dst] = (float)host[pe + src];
-                if (gdY) gdY[dst] = (float)host[2 * pe + src];
-                z += host[3 * pe + src];
-            }
-        if (gz) gz[i] = (float)z;
-        cell_off += (size_t)g.H * g.W;
+        const size_t pe = (size_t)b->h_tubes[i].plane, cells_i = (size_t)g.H * g.W;
+        float* const out[3] = {gdP, gdX, gdY};
+        for (int k = 0; k < 3; ++k)
+            if (out[k])
+                ck(cudaMemcpyAsync(out[k] + cell_off, adj[i].lam[0] + k * pe, cells_i * sizeof(float),
+                                   cudaMemcpyDeviceToHost, b->stream),
+                   "read gradients");
+        cell_off += cells_i;
     }
+    std::vector<double> z((size_t)n);
+    for (int i = 0; i < n; ++i)
+        ck(cudaMemcpyAsync(&z[(size_t)i], adj[i].lam[0] + 3 * (size_t)b->h_tubes[i].plane, sizeof(double),
+                           cudaMemcpyDeviceToHost, b->stream),
+           "read gradients");
+    ck(cudaStreamSynchronize(b->stream), "gradients sync");
+    for (int i = 0; i < n; ++i)
+        if (gz) gz[i] = (float)z[(size_t)i];
     for (int i = 0; i < n; ++i) {
         b->h_tubes[i].hist = nullptr;
         b->h_tubes[i].tmm_hist = nullptr;

@@ -336,6 +336,11 @@ int adjoint_strip_blocks(int strips);                   // CTAs those strips tak
 // two-mass state into slot 0 of tmm_hist).
 cudaError_t launch_history_seed(const TubeDev* tubes, int ntubes, int max_plane_cells, int par, cudaStream_t stream);
 
+// After the sweep: each tube's gradient frames as unpadded floats in the first
+// three planes of AdjTube::lam[0], its z_inv gradient as a double at the fourth.
+cudaError_t launch_gradients_out(const TubeDev* tubes, const AdjTube* adj, int ntubes, int max_plane_cells,
+                                 cudaStream_t stream);
+
 // ---- device map builder (vs_mapbuild.cu) ------------------------------------
 enum : int { MAP_DEPTH_NONE = 0, MAP_DEPTH_CIRCLE = 1, MAP_DEPTH_ELLIPSE = 2 };
 

@@ -52,7 +52,7 @@ bool resident_plan(const TubeGrid* grids, int n, int npairs, bool fast, Resident
     std::vector<int> idx((size_t)n);
     std::vector<double> t((size_t)n);
     double best = 1e300;
-    for (int C : {1, 2, 3, 4, 6, 8, 12, 16}) {
+    for (int C : {1, 2, 3, 4, 6, 8, 16}) {
         ResidentPlan p;
         p.ctas = C;
         p.fast = fast;
