@@ -640,7 +640,8 @@ def run_b200(args, rank, world):
                 "parallelism": (f"LPT tube sharding of one {args.tubes}-tube batch x{world} (no collective)"
                                 if args.strong else f"tube sharding x{world} (no collective)"),
                 "arithmetic": "reciprocal form (fast_math=1)" if fast else "reference rounding (fast_math=0)",
-                "l2": "state + maps per GPU > 126 MB L2 and 33075 launches per timed step; no flush"},
+                "l2": ("state + maps per GPU > 126 MB L2, read once per timed step; no flush" if whole else
+                       "state + maps per GPU > 126 MB L2 and 33075 launches per timed step; no flush")},
         "roofline": {"bound": "on-chip latency" if whole else "hbm", "achieved": round(achieved_gbs, 1), "peak": peak, "unit": "GB/s",
                      "frac": round(achieved_gbs / peak, 4), "traffic": prof["traffic"],
                      # DRAM bytes the launch really moves (ncu, same kernel and workload) per
