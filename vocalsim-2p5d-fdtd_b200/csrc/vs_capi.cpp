@@ -210,6 +210,18 @@ struct vs_solver {
 namespace vsb {
 namespace {
 
+// Host to device on the batch's stream.  The stream does not wait for the
+// default stream, so what a kernel on it reads is written by copies and fills
+// on the same stream: a plain cudaMemcpy or cudaMemset may still be under way
+// when the kernel starts.  The sources are pageable, and staged at return.
+void to_device(const vs_batch* b, void* dst, const void* src, size_t bytes, const char* what) {
+    ck(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, b->stream), what);
+}
+
+void upload_tubes(const vs_batch* b) {
+    to_device(b, b->d_tubes, b->h_tubes.data(), b->h_tubes.size() * sizeof(TubeDev), "upload tube descriptors");
+}
+
 // Default launch shapes when no autotune ran: 16-row strips with 4 warps per
 // CTA, and 4-row strips with 2 warps per CTA below kSmallGridCells cells;
 // with fast_math the quad strips of the same heights (16 rows x 4 warps,
@@ -270,15 +282,12 @@ void upload_sources(vs_batch* b, int64_t need) {
         TubeDev& t = b->h_tubes[i];
         if (g.tmm) { t.src = nullptr; t.src_len = 0; b->src_len[i] = INT64_MAX; continue; }
         float* dst = (float*)((char*)b->src_arena + off[i]);
-        if (upload[i])
-            ck(cudaMemcpy(dst, g.source.data(), g.source.size() * sizeof(float), cudaMemcpyHostToDevice),
-               "upload source table");
+        if (upload[i]) to_device(b, dst, g.source.data(), g.source.size() * sizeof(float), "upload source table");
         t.src = dst;
         t.src_len = (int64_t)g.source.size();
         b->src_len[i] = t.src_len;
     }
-    ck(cudaMemcpy(b->d_tubes, b->h_tubes.data(), b->h_tubes.size() * sizeof(TubeDev),
-                  cudaMemcpyHostToDevice), "upload tube descriptors");
+    upload_tubes(b);
 }
 
 // Largest dynamic shared memory a CTA may use on this device.
@@ -411,7 +420,8 @@ Tile* make_tiles(vs_batch* b, int shape, int* n) {
     }
     Tile* d = nullptr;
     ck(cudaMalloc(&d, tiles.size() * sizeof(Tile)), "cudaMalloc(tiles)");
-    const cudaError_t e = cudaMemcpy(d, tiles.data(), tiles.size() * sizeof(Tile), cudaMemcpyHostToDevice);
+    const cudaError_t e = cudaMemcpyAsync(d, tiles.data(), tiles.size() * sizeof(Tile), cudaMemcpyHostToDevice,
+                                          b->stream);
     if (e != cudaSuccess) cudaFree(d);
     ck(e, "upload tiles");
     *n = (int)tiles.size();
@@ -427,7 +437,7 @@ void ensure_third_set(vs_batch* b) {
     for (const TubeDev& t : b->h_tubes) total += 3 * (size_t)t.plane * sizeof(float) + slots;
     total += kGuard;
     ck(cudaMalloc(&b->x_mem, total), "cudaMalloc(third state set)");
-    ck(cudaMemset(b->x_mem, 0, total), "zero third state set");
+    ck(cudaMemsetAsync(b->x_mem, 0, total, b->stream), "zero third state set");
     b->x_bytes = total;
     size_t off = kGuard;
     for (TubeDev& t : b->h_tubes) {
@@ -437,8 +447,7 @@ void ensure_third_set(vs_batch* b) {
         t.tmm64_x = reinterpret_cast<TmmState64*>(b->x_mem + off + align_up(sizeof(TmmState)));
         off += slots;
     }
-    ck(cudaMemcpy(b->d_tubes, b->h_tubes.data(), b->h_tubes.size() * sizeof(TubeDev), cudaMemcpyHostToDevice),
-       "upload tube descriptors");
+    upload_tubes(b);
 }
 
 void build_tiles(vs_batch* b, int shape) {
@@ -741,21 +750,19 @@ void upload_static_tube(vs_batch* b, size_t i) {
             std::fill(buf.begin(), buf.end(), 0.0f);
             for (int r = 0; r < g.H; ++r)
                 std::memcpy(&buf[(size_t)r * g.pitch], &src[(size_t)r * g.W], g.W * sizeof(float));
-            ck(cudaMemcpy((void*)dst, buf.data(), pl * sizeof(float), cudaMemcpyHostToDevice), "upload depth");
+            to_device(b, (void*)dst, buf.data(), pl * sizeof(float), "upload depth");
         };
         up(g.dP, t.dP);
         up(g.dX, t.dX);
         up(g.dY, t.dY);
-        ck(cudaMemcpy((void*)t.code, g.code.data(), g.code.size(), cudaMemcpyHostToDevice), "upload codes");
+        to_device(b, (void*)t.code, g.code.data(), g.code.size(), "upload codes");
         if (b->desc) {
             std::vector<uint8_t> desc;
             std::vector<float> ta, tb;
             build_descriptors(g, desc, ta, tb, &b->h_tubes[i].ndesc, !b->fast);
-            ck(cudaMemcpy((void*)t.desc, desc.data(), desc.size(), cudaMemcpyHostToDevice), "upload descriptors");
-            ck(cudaMemcpy((void*)t.desc_a, ta.data(), ta.size() * sizeof(float), cudaMemcpyHostToDevice),
-               "upload descriptor table");
-            ck(cudaMemcpy((void*)t.desc_b, tb.data(), tb.size() * sizeof(float), cudaMemcpyHostToDevice),
-               "upload descriptor table");
+            to_device(b, (void*)t.desc, desc.data(), desc.size(), "upload descriptors");
+            to_device(b, (void*)t.desc_a, ta.data(), ta.size() * sizeof(float), "upload descriptor table");
+            to_device(b, (void*)t.desc_b, tb.data(), tb.size() * sizeof(float), "upload descriptor table");
         }
     }
 }
@@ -830,12 +837,10 @@ void upload_static(vs_batch* b) {
         const char* base = reinterpret_cast<const char*>(t.dP);
         // a device-built tube's image starts at its descriptors
         const size_t from = b->grids[i].device_maps ? (size_t)(reinterpret_cast<const char*>(t.desc) - base) : 0;
-        ck(cudaMemcpy((void*)(base + from), img[i].data() + from, img[i].size() - from, cudaMemcpyHostToDevice),
-           "upload maps");
+        to_device(b, (void*)(base + from), img[i].data() + from, img[i].size() - from, "upload maps");
     }
     // the descriptor counts (TubeDev::ndesc) are known now
-    ck(cudaMemcpy(b->d_tubes, b->h_tubes.data(), n * sizeof(TubeDev), cudaMemcpyHostToDevice),
-       "upload tube descriptors");
+    upload_tubes(b);
 }
 
 void reset_state(vs_batch* b) {
@@ -849,6 +854,14 @@ void reset_state(vs_batch* b) {
     ck(cudaMemcpyAsync(b->d_rs, &rs, sizeof(rs), cudaMemcpyHostToDevice, b->stream), "reset run state");
     ck(cudaStreamSynchronize(b->stream), "reset sync");
     b->step = 0;
+}
+
+// The resident plan's tube order (made with the default shape).
+void upload_order(vs_batch* b) {
+    const std::vector<int>& order = b->resident.order;
+    if (order.empty()) return;
+    ck(cudaMalloc(&b->d_order, order.size() * sizeof(int)), "cudaMalloc(tube order)");
+    to_device(b, b->d_order, order.data(), order.size() * sizeof(int), "upload tube order");
 }
 
 void create_batch(int n, const vs_params* params, const vs_geometry* geoms, vs_batch* b) {
@@ -943,20 +956,15 @@ void create_batch(int n, const vs_params* params, const vs_geometry* geoms, vs_b
     upload_sources(b, need);
     build_maps_on_device(b);
     upload_static(b);
-    reset_state(b);
     // small grids (a single tube) need short strips to spread over the SMs
     b->shape = default_shape(b);
+    upload_order(b);
+    reset_state(b);                        // waits for the uploads
 }
 
 // `count` steps of every tube on the resident kernel.
 void issue_resident(vs_batch* b, int64_t count, bool hist) {
-    const ResidentPlan& plan = b->resident;
-    if (!b->d_order) {
-        ck(cudaMalloc(&b->d_order, plan.order.size() * sizeof(int)), "cudaMalloc(tube order)");
-        ck(cudaMemcpy(b->d_order, plan.order.data(), plan.order.size() * sizeof(int), cudaMemcpyHostToDevice),
-           "upload tube order");
-    }
-    ck(launch_resident_run(b->d_tubes, b->d_rs, b->d_order, count, plan, b->stream, hist), "resident launch");
+    ck(launch_resident_run(b->d_tubes, b->d_rs, b->d_order, count, b->resident, b->stream, hist), "resident launch");
 }
 
 // Issue `count` steps from the device step counter (graph chunks of kChunk
@@ -1471,14 +1479,14 @@ void run_adjoint(vs_batch* b, const float* gtrace, float* gdP, float* gdX, float
         ck(cudaMemcpyAsync(&z[(size_t)i], adj[i].lam[0] + 3 * (size_t)b->h_tubes[i].plane, sizeof(double),
                            cudaMemcpyDeviceToHost, b->stream),
            "read gradients");
-    ck(cudaStreamSynchronize(b->stream), "gradients sync");
-    for (int i = 0; i < n; ++i)
-        if (gz) gz[i] = (float)z[(size_t)i];
     for (int i = 0; i < n; ++i) {
         b->h_tubes[i].hist = nullptr;
         b->h_tubes[i].tmm_hist = nullptr;
     }
-    ck(cudaMemcpy(b->d_tubes, b->h_tubes.data(), n * sizeof(TubeDev), cudaMemcpyHostToDevice), "restore descriptors");
+    upload_tubes(b);
+    ck(cudaStreamSynchronize(b->stream), "gradients sync");
+    for (int i = 0; i < n; ++i)
+        if (gz) gz[i] = (float)z[(size_t)i];
     b->step = steps;
 }
 
@@ -1553,16 +1561,13 @@ void section_setup(vs_batch* b) {
         t.ds = (double)g.dims.ds;
         t.pivot = (int64_t)g.dims.tube_mid_y * g.W + g.dims.tube_end_x;
         t.H = g.H; t.W = g.W; t.nsec = (int32_t)ns;
-        ck(cudaMemcpy(dcx, cx[i].data(), cells * sizeof(SectionCell), cudaMemcpyHostToDevice), "upload section cells");
-        ck(cudaMemcpy(dcx + cells, cy[i].data(), cells * sizeof(SectionCell), cudaMemcpyHostToDevice),
-           "upload section cells");
+        to_device(b, dcx, cx[i].data(), cells * sizeof(SectionCell), "upload section cells");
+        to_device(b, dcx + cells, cy[i].data(), cells * sizeof(SectionCell), "upload section cells");
         std::vector<double> w0(g.major_m.begin(), g.major_m.end());
-        ck(cudaMemcpy(const_cast<double*>(t.w0), w0.data(), ns * sizeof(double), cudaMemcpyHostToDevice),
-           "upload nominal widths");
+        to_device(b, const_cast<double*>(t.w0), w0.data(), ns * sizeof(double), "upload nominal widths");
     }
     ck(cudaMalloc(&b->d_sec, n * sizeof(SectionTube)), "cudaMalloc(section descriptors)");
-    ck(cudaMemcpy(b->d_sec, b->h_sec.data(), n * sizeof(SectionTube), cudaMemcpyHostToDevice),
-       "upload section descriptors");
+    to_device(b, b->d_sec, b->h_sec.data(), n * sizeof(SectionTube), "upload section descriptors");
 }
 
 void set_sections(vs_batch* b, const double* width, const double* depth, const double* zinv) {
@@ -1646,8 +1651,8 @@ void set_maps(vs_batch* b, int i, const float* dP, const float* dX, const float*
     b->h_tubes[i].zinv = zinv;
     upload_static_tube(b, (size_t)i);
     b->sec_maps = false;
-    ck(cudaMemcpy(b->d_tubes, b->h_tubes.data(), b->h_tubes.size() * sizeof(TubeDev), cudaMemcpyHostToDevice),
-       "upload tube descriptors");
+    upload_tubes(b);
+    ck(cudaStreamSynchronize(b->stream), "maps sync");
     b->ck_steps = 0;    // checkpoints no longer match the maps
 }
 

@@ -797,6 +797,12 @@ resident_kernel(const TubeDev* __restrict__ tubes, RunState* __restrict__ rs,
     X.C = (int)cluster.num_blocks();
     X.k = (int)cluster.block_rank();
     X.tube = order[blockIdx.y];
+    // no address is formed from an index outside the batch; the whole cluster
+    // reads the same one, so it leaves together
+    if ((unsigned)X.tube >= gridDim.y) {
+        if (threadIdx.x == 0) atomicExch(&rs->error, VS_ERR_CUDA);
+        return;
+    }
     X.T = tubes + X.tube;
     X.rs = rs;
     X.sm = res_smem;
