@@ -265,11 +265,13 @@ int vs_batch_set_adjoint_form(vs_batch* b, int32_t form);
 int vs_batch_set_adjoint_rows(vs_batch* b, int32_t rows);
 
 /* Failure-path hook, no counterpart in the reference: the number of polls a
- * kernel's wait for its bulk row copies (band and staged quad-strip shapes)
- * makes before it gives up, and the run returns VS_ERR_TIMEOUT with the
- * state not valid; 0 restores the default (2^22).  A kernel that gives up
- * still waits, with the default limit, for its own copies in flight before it
- * exits.  Tests lower it to drive the timeout path without a fault. */
+ * kernel's wait makes before it gives up, and the run returns VS_ERR_TIMEOUT
+ * with the state not valid; 0 restores the default (2^22).  It covers the
+ * waits for bulk row copies (band and staged quad-strip shapes) and the cluster
+ * shape's waits for its neighbours' rows and the two-mass flow, so also the
+ * default shape of most batches.  A kernel that gives up still waits, with a
+ * limit of its own, for its copies and its neighbours' stores in flight before
+ * it exits.  Tests lower it to drive the timeout path without a fault. */
 int vs_batch_set_wait_limit(vs_batch* b, uint32_t polls);
 
 /* Time every compiled tile shape on `steps` steps and keep the fastest.  The

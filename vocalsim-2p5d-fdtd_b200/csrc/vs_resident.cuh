@@ -205,6 +205,7 @@ __host__ __device__ constexpr int rec_bytes(bool exact) { return rec_desc(exact)
 constexpr int kEdgeP = kMaxRows;
 constexpr int kEdgeFloats = 2 * kMaxRows + 4;
 
+constexpr int kDrainPolls = 1 << 14;             // about 2 ms; a store into a neighbour takes about 1 us
 constexpr int kHashSlots = 1024;
 constexpr int kMaxPairs = 128;                   // descriptor pairs of a tube (vowel tubes: 50 to 75)
 constexpr int kTab = kMaxPairs * 16;             // one table of 16-byte entries
@@ -216,7 +217,9 @@ constexpr int kOffBar = 0, kOffFail = 16, kOffM1 = 32;
 // two-mass source: excitation values in flight (more than the largest cluster has CTAs), the excitation
 // cell's P' by step parity
 constexpr int kExeRing = 32;
-constexpr int kOffRing = 64, kOffWord = kOffRing + 8 * kExeRing, kOffTab = kOffWord + 16;
+constexpr int kOffRing = 64, kOffWord = kOffRing + 8 * kExeRing;
+// by CTA of the cluster: the exchanges it sent if it gave up, else the steps of the launch
+constexpr int kMaxCtas = 16, kOffSent = kOffWord + 16, kOffTab = kOffSent + 4 * kMaxCtas;
 __host__ __device__ constexpr int off_ghost(bool exact) { return kOffTab + (exact ? 8 : 4) * kTab; }
 
 struct ResLayout {
@@ -705,7 +708,7 @@ __device__ __forceinline__ void run_tile(const TileCtx& X) {
         step_sync(32 * X.nw);
         // a wait that ran out in this step: every warp sees it after this barrier
         if (sfail[p]) {
-            for (int i = 0; i < 64; ++i) __nanosleep(1000);     // stores in flight land before the CTAs meet
+            if (threadIdx.x == 0) sfail[2] = min(m + 1, nsteps - 1);      // exchanges sent, see drain_exchange
             break;
         }
     }
@@ -784,6 +787,34 @@ __device__ __noinline__ void run_two_mass(const TileCtx& X, bool hist) {
     else
         two_mass_loop(X, T->tmm, th, [&](const TmmState& s) { return tmm_prepare(T->tmmc, s); },
                       [](const TmmPrep& o, TmmState& s, float p) { return tmm_finish(o, s, p); });
+}
+
+// Waits until every byte the neighbour CTAs have sent to this one has landed,
+// so that it can leave: after a wait ran out, stores may still be under way.
+// Called by one thread once no CTA of the cluster sends any more.  own, up,
+// dn: the exchanges this CTA and its neighbours made (each arrived once on the
+// barrier of its parity here with `expect` bytes, and sent from_up or from_dn
+// bytes there).  A barrier with E arrivals and R bytes landed has the tx-count
+// E expect - R, its phases end where that is 0, and E or E - 1 of them have
+// ended (an arrival follows the wait for the phase before it).  With T the
+// bytes sent, E expect - T is taken off and a guard of 1 added, which leaves
+// the count at 1 + T - R > 0: no phase ends from here on, so whether the
+// last one has can be tested; if so, one more arrival opens the next phase's
+// end.  Without the guard that phase ends when R = T.  Bounded like every wait.
+__device__ __noinline__ void drain_exchange(uint64_t* bar, int par0, int expect, int from_up, int from_dn, int own,
+                                            int up, int dn) {
+    for (int p = 0; p < 2; ++p) {
+        auto count = [&](int sent) { return (sent + (((par0 + 1) & 1) == p)) / 2; };    // of parity p
+        const int E = count(own);
+        const int more = from_up * count(up) + from_dn * count(dn) - E * expect + 1;
+        if (more > 0) mbar_tx_more(bar + p, (uint32_t)more);
+        if (more < 0) mbar_tx_less(bar + p, (uint32_t)-more);
+        const bool ended = E == 0 || mbar_test(bar + p, (uint32_t)(E - 1) & 1u);
+        if (ended) mbar_arrive(bar + p);
+        mbar_tx_less(bar + p, 1);
+        const uint32_t phase = (uint32_t)(ended ? E : E - 1) & 1u;
+        for (int i = 0; i < kDrainPolls && !mbar_test(bar + p, phase); ++i) __nanosleep(100);
+    }
 }
 
 template <bool HIST, bool EXACT, bool TMM>
@@ -963,6 +994,7 @@ resident_kernel(const TubeDev* __restrict__ tubes, RunState* __restrict__ rs,
             mbar_fence_init();
             int* f = reinterpret_cast<int*>(res_smem + kOffFail);
             f[0] = f[1] = 0;
+            for (int i = 0; i < kMaxCtas; ++i) reinterpret_cast<int*>(res_smem + kOffSent)[i] = nsteps;
             u64* w = reinterpret_cast<u64*>(res_smem + kOffRing);
             for (int i = 0; i < kExeRing + 2; ++i) w[i] = ~0ull << 32;      // tag: no step
         }
@@ -985,8 +1017,23 @@ resident_kernel(const TubeDev* __restrict__ tubes, RunState* __restrict__ rs,
     }
     __syncthreads();
     const int* f = reinterpret_cast<const int*>(res_smem + kOffFail);
-    if (tid == 0 && (f[0] | f[1])) atomicExch(&rs->error, VS_ERR_TIMEOUT);
-    cluster.sync();                                  // no CTA exits while another may store into it
+    int* sent = reinterpret_cast<int*>(res_smem + kOffSent);
+    if (f[0] | f[1]) {
+        if (tid == 0) atomicExch(&rs->error, VS_ERR_TIMEOUT);
+        if (tid < X.C) cluster.map_shared_rank(sent, tid)[X.k] = f[2];
+    }
+    // no CTA exits while another may store into it: without a failure every
+    // store has been waited for by the receiver's last step
+    cluster.sync();
+    if (tid != 0) return;
+    bool failed = false;
+    for (int k = 0; k < X.C; ++k) failed = failed || sent[k] < nsteps;
+    if (!failed) return;
+    auto exchanges = [&](int k) { return k < 0 || k >= X.C ? 0 : min(sent[k], nsteps - 1); };
+    const int from_up = X.k > 0 ? 16 * lanes : 0, from_dn = X.k + 1 < X.C ? 8 * lanes : 0;
+    if (from_up + from_dn > 0)
+        drain_exchange(reinterpret_cast<uint64_t*>(res_smem + kOffBar), (int)(rs->step & 1), from_up + from_dn, from_up, from_dn,
+                       exchanges(X.k), exchanges(X.k - 1), exchanges(X.k + 1));
 }
 
 }  // namespace
