@@ -343,7 +343,10 @@ int vs_batch_get_maps(const vs_batch* b, int32_t tube, int32_t* cell_type, float
 int vs_batch_get_fields(const vs_batch* b, int32_t tube, float* p, float* vx, float* vy);
 
 /* Forward `steps` steps from rest, keeping a state checkpoint every
- * ckpt_every steps for vs_batch_adjoint; traces (host, n x steps) may be NULL. */
+ * ckpt_every steps for vs_batch_adjoint; traces (host, n x steps) may be NULL.
+ * A device wait that gave up is VS_ERR_TIMEOUT, from here or from
+ * vs_batch_adjoint, and leaves no checkpoints; non-finite traces are not
+ * reported. */
 int vs_batch_forward_ckpt(vs_batch* b, int64_t steps, int32_t ckpt_every, float* traces);
 
 /* Gradients of a loss L(traces) given dL/dtrace (host, n x steps of the last

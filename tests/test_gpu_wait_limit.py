@@ -40,3 +40,43 @@ def test_run_reports_the_timeout_and_the_next_run_is_clean(n, model, fast, cuda_
         b.reset()
         np.testing.assert_array_equal(b.run(200), want)
     b.close()
+
+
+@pytest.mark.parametrize("fast", [0, 1])
+@pytest.mark.parametrize("model", MODELS, ids=["float", "double"])
+def test_checkpointed_forward_reports_the_timeout(model, fast, cuda_ok):
+    b = batch(3, fast_math=fast, **model)
+    seed = np.ones((3, 300), np.float32)
+    b.set_wait_limit(1)
+    times_out(lambda: b.forward_ckpt(300, 64))
+    with pytest.raises(V.VsError) as e:              # its checkpoints are not states
+        b.adjoint(seed)
+    assert e.value.status == abi.VS_ERR_INVALID_ARG
+    b.set_wait_limit(0)
+    trace = b.forward_ckpt(300, 64)
+    b.reset()
+    np.testing.assert_array_equal(b.run(300), trace)
+    b.close()
+
+
+@pytest.mark.parametrize("fast", [0, 1])
+@pytest.mark.parametrize("model", MODELS, ids=["float", "double"])
+def test_adjoint_reports_the_timeout(model, fast, cuda_ok):
+    """Several segments: the status of the first recomputed one is kept over those that follow."""
+    b = batch(3, fast_math=fast, **model)
+    seed = np.random.default_rng(1).standard_normal((3, 200)).astype(np.float32)
+    b.forward_ckpt(200, 64)
+    want, want_z = b.adjoint(seed)
+    b.set_wait_limit(1)
+    times_out(lambda: b.adjoint(seed))
+    b.set_wait_limit(0)
+    with pytest.raises(V.VsError) as e:
+        b.adjoint(seed)
+    assert e.value.status == abi.VS_ERR_INVALID_ARG
+    b.forward_ckpt(200, 64)
+    got, got_z = b.adjoint(seed)
+    np.testing.assert_array_equal(got_z, want_z)
+    for x, y in zip(got, want):
+        for u, v in zip(x, y):
+            np.testing.assert_array_equal(u, v)
+    b.close()

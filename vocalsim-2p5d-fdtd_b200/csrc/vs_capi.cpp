@@ -16,6 +16,7 @@
 #include <thread>
 #include <functional>
 #include <cmath>
+#include <cstddef>
 #include <cstring>
 #include <memory>
 #include <new>
@@ -1018,6 +1019,17 @@ void issue_steps(vs_batch* b, int64_t count) {
     }
 }
 
+// After the stream was waited for: the status the device left since the run
+// state was set.  Anything but a non-finite listener sample means that the
+// state is not valid.
+int32_t run_status(const vs_batch* b) {
+    int32_t status = 0;
+    ck(cudaMemcpy(&status, &b->d_rs->error, sizeof(status), cudaMemcpyDeviceToHost), "read run status");
+    if (status != 0 && status != VS_ERR_NONFINITE)
+        throw VsFailure{status, "a bounded device wait gave up; the state is not valid"};
+    return status;
+}
+
 void run_batch(vs_batch* b, int64_t steps, float* traces, int on_device) {
     const int n = (int)b->grids.size();
     if (b->shape < 0) b->shape = default_shape(b);
@@ -1045,10 +1057,7 @@ void run_batch(vs_batch* b, int64_t steps, float* traces, int on_device) {
            "copy traces");
     }
     ck(cudaStreamSynchronize(b->stream), "run sync");
-    int32_t dev_error = 0;
-    ck(cudaMemcpy(&dev_error, &b->d_rs->error, sizeof(dev_error), cudaMemcpyDeviceToHost), "read run status");
-    if (dev_error == VS_ERR_NONFINITE) throw VsFailure{dev_error, "non-finite listener pressure"};
-    if (dev_error != 0) throw VsFailure{dev_error, "a bounded device wait gave up; the state is not valid"};
+    if (run_status(b) == VS_ERR_NONFINITE) throw VsFailure{VS_ERR_NONFINITE, "non-finite listener pressure"};
     if (traces && !on_device) {
         for (int64_t i = 0; i < need; ++i)
             if (!std::isfinite(traces[i])) throw VsFailure{VS_ERR_NONFINITE, "non-finite listener pressure"};
@@ -1089,6 +1098,7 @@ void forward_checkpointed(vs_batch* b, int64_t steps, int every, float* traces, 
         b->trace_cap = need;
     }
     const int count = (int)((steps + every - 1) / every);
+    b->ck_steps = 0;                       // until the states of this forward are known to be valid
     size_t stride = 0;
     for (size_t bytes : b->state_bytes) stride += bytes;
     if (b->ckpt) { cudaFree(b->ckpt); b->ckpt = nullptr; }
@@ -1104,14 +1114,15 @@ void forward_checkpointed(vs_batch* b, int64_t steps, int every, float* traces, 
         issue_steps(b, std::min<int64_t>(every, steps - (int64_t)k * every));
     }
     b->step = steps;
-    b->ck_steps = steps;
-    b->ck_every = every;
-    b->ck_count = count;
     if (traces)
         ck(cudaMemcpyAsync(traces, b->d_trace, need * sizeof(float),
                            traces_on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, b->stream),
            "copy traces");
     ck(cudaStreamSynchronize(b->stream), "forward sync");
+    run_status(b);
+    b->ck_steps = steps;
+    b->ck_every = every;
+    b->ck_count = count;
 }
 
 // Velocities the excitation flow enters, per tube with the two-mass source:
@@ -1416,6 +1427,8 @@ void run_adjoint(vs_batch* b, const float* gtrace, float* gdP, float* gdX, float
     // time split vs_batch_adjoint_times reports
     std::vector<cudaEvent_t> ev(3 * (size_t)b->ck_count, nullptr);
     for (cudaEvent_t& e : ev) ck(cudaEventCreate(&e), "event");
+    const RunState clear{};
+    to_device(b, b->d_rs, &clear, sizeof(clear), "clear run state");
     for (int k = b->ck_count - 1; k >= 0; --k) {
         const int64_t start = (int64_t)k * K;
         const int len = (int)std::min<int64_t>(K, steps - start);
@@ -1426,7 +1439,8 @@ void run_adjoint(vs_batch* b, const float* gtrace, float* gdP, float* gdX, float
         rs.run_start = start;
         rs.trace = b->d_trace;
         rs.trace_stride = len;
-        ck(cudaMemcpyAsync(b->d_rs, &rs, sizeof(rs), cudaMemcpyHostToDevice, b->stream), "set run state");
+        // all but the status, which stays over the segments
+        to_device(b, b->d_rs, &rs, offsetof(RunState, error), "set run state");
         const AdjRun ar{start, len, q};
         ck(cudaMemcpyAsync(b->d_adjrun, &ar, sizeof(ar), cudaMemcpyHostToDevice, b->stream), "set adjoint run");
         ck(cudaEventRecord(ev[3 * k], b->stream), "event");
@@ -1485,9 +1499,12 @@ void run_adjoint(vs_batch* b, const float* gtrace, float* gdP, float* gdX, float
     }
     upload_tubes(b);
     ck(cudaStreamSynchronize(b->stream), "gradients sync");
+    b->step = steps;
+    b->ck_steps = 0;                       // unless the recomputed states are valid
+    run_status(b);
+    b->ck_steps = steps;
     for (int i = 0; i < n; ++i)
         if (gz) gz[i] = (float)z[(size_t)i];
-    b->step = steps;
 }
 
 // The depth kernel's writes of one tube, as autograd.SectionDepthModel lists

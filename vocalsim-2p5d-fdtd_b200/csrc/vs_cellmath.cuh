@@ -357,10 +357,11 @@ __device__ __forceinline__ float pressure_den(float sP, float dp, bool eigen) {
 
 // Listener sample of a step; a non-finite value (an unstable tube) also
 // raises the run's sticky error word, so runs that keep their traces on the
-// device report VS_ERR_NONFINITE too.
+// device report VS_ERR_NONFINITE too; it leaves a status that is there, such
+// as a timeout's, in place.
 __device__ __forceinline__ void store_trace(RunState* rs, float* dst, float v) {
     *dst = v;
-    if (!isfinite(v)) atomicExch(&rs->error, VS_ERR_NONFINITE);
+    if (!isfinite(v)) atomicCAS(&rs->error, 0, VS_ERR_NONFINITE);
 }
 
 // Approximate reciprocal (PTX rcp.approx.f32, at most 1 ulp from 1/x).
