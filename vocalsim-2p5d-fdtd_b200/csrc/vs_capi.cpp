@@ -161,6 +161,8 @@ struct vs_batch {
     bool sec_maps = false;                 // the maps on the device came from set_sections
     cudaGraphExec_t hist_graph = nullptr;  // ck_every history steps
     cudaGraphExec_t adj_graph = nullptr;   // ck_every reverse steps
+    int hist_graph_len = 0;
+    int hist_graph_steps = 0;              // time steps of one of its launches
     int adj_graph_len = 0;
     int adj_graph_form = -1;
     float adj_recompute_ms = 0.0f;         // device time of the last adjoint's recomputation / reverse steps
@@ -768,9 +770,6 @@ void upload_static_tube(vs_batch* b, size_t i) {
     }
 }
 
-// Every tube's read-only block (depth planes, codes, fast_math descriptors
-// and tables, from TubeDev::dP on, as laid out in the arena), staged on the
-// host in parallel and copied with one transfer per tube.
 // Distinct descriptors of two adjacent cells (even column first), the count
 // the resident kernel's tables are sized for.
 int descriptor_pairs(const TubeGrid& g, const std::vector<uint8_t>& desc) {
@@ -787,6 +786,9 @@ int descriptor_pairs(const TubeGrid& g, const std::vector<uint8_t>& desc) {
     return n;
 }
 
+// Every tube's read-only block (depth planes, codes, fast_math descriptors
+// and tables, from TubeDev::dP on, as laid out in the arena), staged on the
+// host in parallel and copied with one transfer per tube.
 void upload_static(vs_batch* b) {
     const size_t n = b->grids.size();
     std::vector<std::vector<char>> img(n);
@@ -1391,7 +1393,7 @@ void run_adjoint(vs_batch* b, const float* gtrace, float* gdP, float* gdX, float
     int64_t cells = 0;
     for (const TubeGrid& g : b->grids) cells += (int64_t)(g.H - 2) * (g.W - 2);
     const int hshape = history_shape(cells, b->fast);
-    if (!b->d_hist_tiles) b->d_hist_tiles = make_tiles(b, hshape, &b->n_hist_tiles);
+    if (!hist_cluster && !b->d_hist_tiles) b->d_hist_tiles = make_tiles(b, hshape, &b->n_hist_tiles);
     auto hist_step = [&](int j) {
         return launch_step_history(hshape, b->d_tubes, b->d_hist_tiles, b->n_hist_tiles, b->d_rs, j, b->stream);
     };
@@ -1413,10 +1415,14 @@ void run_adjoint(vs_batch* b, const float* gtrace, float* gdP, float* gdX, float
         return launch_adjoint_step(b->d_tubes, b->d_adj, n, max_tiles, b->d_adjrun, local, j, b->stream,
                                    two ? ADJ_FORM_STRIPS : form, rows);
     };
-    if (b->adj_graph_len != K || b->adj_graph_form != form || b->adj_graph_rows != rows || !b->hist_graph ||
-        !b->adj_graph) {
+    const int hist_steps = hist_two ? 2 : 1;
+    if (!hist_cluster && (b->hist_graph_len != K || b->hist_graph_steps != hist_steps || !b->hist_graph)) {
         if (hist_two) capture(b, &b->hist_graph, "capture history steps", hist2_step, K / 2);
         else capture(b, &b->hist_graph, "capture history steps", hist_step, K);
+        b->hist_graph_len = K;
+        b->hist_graph_steps = hist_steps;
+    }
+    if (b->adj_graph_len != K || b->adj_graph_form != form || b->adj_graph_rows != rows || !b->adj_graph) {
         capture(b, &b->adj_graph, "capture reverse steps", [&](int j) { return adj_launch(j, K); }, launches(K));
         b->adj_graph_len = K;
         b->adj_graph_form = form;
