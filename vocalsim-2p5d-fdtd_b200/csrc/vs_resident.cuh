@@ -252,12 +252,28 @@ struct TileCtx {
     bool tmm;                 // two-mass source
 };
 
+// a / b for b = -nb and y = 1 / b correctly rounded, in double: the quotient of
+// two floats lies at least 2^-50 of itself away from every value half-way
+// between two floats (subnormal ones too) that it does not equal, so a double
+// quotient good to an ulp rounds to the IEEE float quotient.  y refined once is
+// good to 2^-47, the quotient corrected by its residual to an ulp of the double.
+__device__ __forceinline__ float quotient_by_double(float a, float nb, float y) {
+    const double d = nb, y0 = y, n = a;
+    const double y1 = __fma_rn(y0, __fma_rn(d, y0, 1.0), y0);
+    const double q = __dmul_rn(n, y1);
+    return __double2float_rn(__fma_rn(__fma_rn(d, q, n), y1, q));
+}
+
 // a[k] / b[k] for N pairs, correctly rounded: nb = -b, y = 1 / b correctly
 // rounded (0 where the result is 0 by definition: ring and no-pressure cells).
 // Two fused corrections of a y (P. Markstein, IBM J. Res. Dev. 34(1), 1990) give
-// the IEEE quotient while nothing on the way leaves the normal range; a warp
-// that meets a numerator outside 2^-80 .. 2^100 (the first steps of a wave
-// front) divides the block again with the IEEE division.
+// the IEEE quotient while nothing on the way leaves the normal range, which
+// holds for numerators of 2^-80 .. 2^100 and denominators of 2^-26 .. 2^46.  A
+// warp that meets a smaller numerator (the wave front of a run's first steps,
+// which stretches over most of the frame) forms the block's quotients in
+// double; one that meets a larger numerator divides.  Steps 128 to 512 from rest of 256 tubes: 122 us a
+// step when such blocks divided, 28 in double, 18 past the front (two-step
+// strips, which divide: 57).
 template <int N>
 __device__ __forceinline__ void quotients(u64 (&a)[N], const u64 (&nb)[N], const u64 (&y)[N]) {
     u64 q[N], r[N];
@@ -273,11 +289,17 @@ __device__ __forceinline__ void quotients(u64 (&a)[N], const u64 (&nb)[N], const
     static_for<0, N>([&](auto kc) { q[kc] = fma2(r[kc], y[kc], q[kc]); });
     static_for<0, N>([&](auto kc) { r[kc] = fma2(nb[kc], q[kc], a[kc]); });
     static_for<0, N>([&](auto kc) { q[kc] = fma2(r[kc], y[kc], q[kc]); });
-    if (__any_sync(0xffffffffu, odd || top > 1.2676506e30f)) {
-        auto div = [](float v, float nd, float rc) { return rc == 0.0f ? 0.0f : fdiv_z(v, -nd); };
-        static_for<0, N>([&](auto kc) {
-            q[kc] = pk(div(plo(a[kc]), plo(nb[kc]), plo(y[kc])), div(phi(a[kc]), phi(nb[kc]), phi(y[kc])));
-        });
+    const bool large = top > 1.2676506e30f;
+    if (__any_sync(0xffffffffu, odd || large)) {
+        auto each = [&](auto&& div) {
+            static_for<0, N>([&](auto kc) {
+                const float y0 = plo(y[kc]), y1 = phi(y[kc]);
+                q[kc] = pk(y0 == 0.0f ? 0.0f : div(plo(a[kc]), plo(nb[kc]), y0),
+                           y1 == 0.0f ? 0.0f : div(phi(a[kc]), phi(nb[kc]), y1));
+            });
+        };
+        if (__any_sync(0xffffffffu, large)) each([](float v, float nd, float) { return fdiv_z(v, -nd); });
+        else each([](float v, float nd, float rc) { return quotient_by_double(v, nd, rc); });
     }
     static_for<0, N>([&](auto kc) { a[kc] = q[kc]; });
 }
