@@ -213,7 +213,7 @@ constexpr int kTab = kMaxPairs * 16;             // one table of 16-byte entries
 // (al_x, al_y), (zo_x, -zi_x), (zo_y, -zi_y).  Reference arithmetic: (-sP, -), (-den_x, 1 / den_x),
 // (-den_y, 1 / den_y), (mB_x, -mS_x), (A_x, B_x), (mB_y, -mS_y), (A_y, B_y), (W_x, W_y); the wall term's
 // pressure is A Pc + B Pn.
-constexpr int kOffBar = 0, kOffFail = 16, kOffM1 = 32;
+constexpr int kOffBar = 0, kOffFail = 16, kOffTop = 28, kOffM1 = 32;     // kOffTop: see quotients()
 // two-mass source: excitation values in flight (more than the largest cluster has CTAs), the excitation
 // cell's P' by step parity
 constexpr int kExeRing = 32;
@@ -271,14 +271,14 @@ __device__ __forceinline__ float quotient_by_double(float a, float nb, float y) 
 // holds for numerators of 2^-80 .. 2^100 and denominators of 2^-26 .. 2^46.  A
 // warp that meets a smaller numerator (the wave front of a run's first steps,
 // which stretches over most of the frame) forms the block's quotients in
-// double; one that meets a larger numerator divides.  Steps 128 to 512 from rest of 256 tubes: 122 us a
+// double; one that meets a larger numerator, or a tube with another denominator
+// (top = infinity), divides.  Steps 128 to 512 from rest of 256 tubes: 122 us a
 // step when such blocks divided, 28 in double, 18 past the front (two-step
 // strips, which divide: 57).
 template <int N>
-__device__ __forceinline__ void quotients(u64 (&a)[N], const u64 (&nb)[N], const u64 (&y)[N]) {
+__device__ __forceinline__ void quotients(u64 (&a)[N], const u64 (&nb)[N], const u64 (&y)[N], float top) {
     u64 q[N], r[N];
     bool odd = false;
-    float top = 0.0f;
     auto tiny = [](float v) { return (__float_as_uint(v) & 0x7fffffffu) - 1u < 0x17800000u - 1u; };   // 0 < |v| < 2^-80
     static_for<0, N>([&](auto kc) {
         odd = odd || tiny(plo(a[kc])) || tiny(phi(a[kc]));
@@ -303,6 +303,11 @@ __device__ __forceinline__ void quotients(u64 (&a)[N], const u64 (&nb)[N], const
     }
     static_for<0, N>([&](auto kc) { a[kc] = q[kc]; });
 }
+
+// Denominators quotients() takes without dividing (the maps' depths times 1 +
+// sigma, and the velocities' mB + mS: 2^-22 .. 2^20 for every tube built here;
+// a caller's own maps may hold others).
+__device__ __forceinline__ bool plain_den(float b) { return b >= 1.4901161e-8f && b <= 7.0368744e13f; }
 
 // Up to kRegRows rows per group the maps and the pressure and velocity factors
 // stay in registers too; taller groups read them from shared memory.
@@ -497,7 +502,7 @@ __device__ __forceinline__ void run_tile(const TileCtx& X) {
                     if (eigen) static_for<0, N>([&](auto kc) { gf[kc] = diff2(gf[kc], dp[kc], m1); });
                     static_for<0, N>([&](auto kc) { dp[kc] = mul2(P[row[kc]], dp[kc]); });
                     static_for<0, N>([&](auto kc) { sum[kc] = diff2(dp[kc], sum[kc], m1); });
-                    quotients<N>(sum, gf, rp);
+                    quotients<N>(sum, gf, rp, ldsf(sb + kOffTop));
                     static_for<0, N>([&](auto kc) { P[row[kc]] = sum[kc]; });
                     return;
                 }
@@ -640,7 +645,7 @@ __device__ __forceinline__ void run_tile(const TileCtx& X) {
                         nden[kc] = v.x;
                         rec1[kc] = v.y;
                     });
-                    quotients<N>(num, nden, rec1);
+                    quotients<N>(num, nden, rec1, ldsf(sb + kOffTop));
                     static_for<0, N>([&](auto kc) {
                         const ulonglong2 v = tab_at(d[kc], 2);
                         VX[row[kc]] = num[kc];
@@ -648,7 +653,7 @@ __device__ __forceinline__ void run_tile(const TileCtx& X) {
                         nden[kc] = v.x;
                         rec1[kc] = v.y;
                     });
-                    quotients<N>(num, nden, rec1);
+                    quotients<N>(num, nden, rec1, ldsf(sb + kOffTop));
                     static_for<0, N>([&](auto kc) { VY[row[kc]] = num[kc]; });
                     return;
                 }
@@ -884,6 +889,7 @@ resident_kernel(const TubeDev* __restrict__ tubes, RunState* __restrict__ rs,
         for (int e = tid; e < kHashSlots; e += nthr) hash[e] = 0xffffffffu;
         if (tid == 0) {
             *count = 0;
+            *reinterpret_cast<float*>(res_smem + kOffTop) = 0.0f;
             *reinterpret_cast<float2*>(res_smem + kOffM1) = make_float2(-1.0f, -1.0f);
         }
         __syncthreads();
@@ -906,8 +912,9 @@ resident_kernel(const TubeDev* __restrict__ tubes, RunState* __restrict__ rs,
                     dp[h] = dP[o];
                     if constexpr (EXACT) {
                         const float4 a = T->desc_a[id];
-                        if (!(__float_as_uint(a.w) & EXD_PZERO))
-                            rc[h] = fdiv(1.0f, pressure_den(a.x, dp[h], (T->flags & TUBE_EIGEN) != 0));
+                        const float den = pressure_den(a.x, dp[h], (T->flags & TUBE_EIGEN) != 0);
+                        if (!(__float_as_uint(a.w) & EXD_PZERO)) rc[h] = fdiv(1.0f, den);
+                        if (!plain_den(den)) *reinterpret_cast<float*>(res_smem + kOffTop) = INFINITY;
                     } else {
                         rc[h] = rcp_approx(dp[h]);
                     }
@@ -946,6 +953,8 @@ resident_kernel(const TubeDev* __restrict__ tubes, RunState* __restrict__ rs,
                 };
                 auto wb = [z](uint32_t f) { return z && (f & EXD_WALL) && !(f & EXD_WALL_PC) ? -1.0f : 0.0f; };
                 const uint32_t g0 = f0 >> EXD_Y_SHIFT, g1 = f1 >> EXD_Y_SHIFT;
+                if (!plain_den(a0.y) || !plain_den(a1.y) || !plain_den(a0.z) || !plain_den(a1.z))
+                    *reinterpret_cast<float*>(res_smem + kOffTop) = INFINITY;
                 tab[0] = make_float4(-a0.x, -a1.x, 0.0f, 0.0f);
                 tab[kMaxPairs] = make_float4(-a0.y, -a1.y, fdiv(1.0f, a0.y), fdiv(1.0f, a1.y));
                 tab[2 * kMaxPairs] = make_float4(-a0.z, -a1.z, fdiv(1.0f, a0.z), fdiv(1.0f, a1.z));
