@@ -844,6 +844,35 @@ __device__ __noinline__ void drain_exchange(uint64_t* bar, int par0, int expect,
     }
 }
 
+// The end of a launch.  It finds the little it needs again, so that nothing
+// but the kernel's parameters lives through the step loop for it (inlined and
+// with the kernel's variables, it took registers from the loop: one uniform
+// tube 0.86 us a step instead of 0.81, five tubes 12.9 ms instead of 12.3).
+__device__ __noinline__ void leave_cluster(const TubeDev* __restrict__ tubes, RunState* __restrict__ rs,
+                                           const int* __restrict__ order, int nsteps, unsigned char* sm) {
+    cg::cluster_group cluster = cg::this_cluster();
+    const int C = (int)cluster.num_blocks(), k = (int)cluster.block_rank(), tid = threadIdx.x;
+    const int* f = reinterpret_cast<const int*>(sm + kOffFail);
+    int* sent = reinterpret_cast<int*>(sm + kOffSent);
+    __syncthreads();
+    if (f[0] | f[1]) {
+        if (tid == 0) atomicExch(&rs->error, VS_ERR_TIMEOUT);
+        if (tid < C) cluster.map_shared_rank(sent, tid)[k] = f[2];
+    }
+    // no CTA exits while another may store into it: without a failure every
+    // store has been waited for by the receiver's last step
+    cluster.sync();
+    bool failed = false;
+    for (int i = 0; i < C; ++i) failed = failed || sent[i] < nsteps;
+    if (tid != 0 || !failed) return;
+    const int lanes = ((tubes[order[blockIdx.y]].W - 2) / kTileCols + 1) * 32;
+    auto exchanges = [&](int i) { return i < 0 || i >= C ? 0 : min(sent[i], nsteps - 1); };
+    const int from_up = k > 0 ? 16 * lanes : 0, from_dn = k + 1 < C ? 8 * lanes : 0;
+    if (from_up + from_dn > 0)
+        drain_exchange(reinterpret_cast<uint64_t*>(sm + kOffBar), (int)(rs->step & 1), from_up + from_dn, from_up, from_dn,
+                       exchanges(k), exchanges(k - 1), exchanges(k + 1));
+}
+
 template <bool HIST, bool EXACT, bool TMM>
 __global__ void __launch_bounds__(kMaxWarps * 32, 1)
 resident_kernel(const TubeDev* __restrict__ tubes, RunState* __restrict__ rs,
@@ -1046,25 +1075,7 @@ resident_kernel(const TubeDev* __restrict__ tubes, RunState* __restrict__ rs,
     } else {
         run_idle(X);
     }
-    __syncthreads();
-    const int* f = reinterpret_cast<const int*>(res_smem + kOffFail);
-    int* sent = reinterpret_cast<int*>(res_smem + kOffSent);
-    if (f[0] | f[1]) {
-        if (tid == 0) atomicExch(&rs->error, VS_ERR_TIMEOUT);
-        if (tid < X.C) cluster.map_shared_rank(sent, tid)[X.k] = f[2];
-    }
-    // no CTA exits while another may store into it: without a failure every
-    // store has been waited for by the receiver's last step
-    cluster.sync();
-    if (tid != 0) return;
-    bool failed = false;
-    for (int k = 0; k < X.C; ++k) failed = failed || sent[k] < nsteps;
-    if (!failed) return;
-    auto exchanges = [&](int k) { return k < 0 || k >= X.C ? 0 : min(sent[k], nsteps - 1); };
-    const int from_up = X.k > 0 ? 16 * lanes : 0, from_dn = X.k + 1 < X.C ? 8 * lanes : 0;
-    if (from_up + from_dn > 0)
-        drain_exchange(reinterpret_cast<uint64_t*>(res_smem + kOffBar), (int)(rs->step & 1), from_up + from_dn, from_up, from_dn,
-                       exchanges(X.k), exchanges(X.k - 1), exchanges(X.k + 1));
+    leave_cluster(tubes, rs, order, nsteps, res_smem);
 }
 
 }  // namespace
