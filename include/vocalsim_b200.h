@@ -240,7 +240,9 @@ int vs_batch_set_stream(vs_batch* b, void* cuda_stream);
  * coupled wall oscillator keeps its state on its own thread-block cluster (up
  * to 16 CTAs, halo rows exchanged through distributed shared memory) and runs
  * every step of a vs_batch_run / vs_run call in one launch.  It is the default
- * wherever the tubes fit its registers and shared memory. */
+ * wherever the tubes fit its registers and shared memory; runs of up to four
+ * steps of a default batch that fills the GPU take the step kernels, whose
+ * values are the same. */
 int vs_batch_set_tile(vs_batch* b, int32_t tile_index);
 
 /* Device time of the last vs_batch_adjoint call, split into the segments'

@@ -112,6 +112,7 @@ struct vs_batch {
     cudaStream_t stream = nullptr;
     bool own_stream = false;
     int shape = -1;                        // chosen tile shape (-1 = not chosen)
+    bool default_run = true;               // the shape is the default choice, not the caller's or the autotuner's
     cudaGraphExec_t graph = nullptr;
     int graph_shape = -1;
     int64_t step = 0;                      // host mirror of RunState::step
@@ -357,17 +358,36 @@ int single_step_shape(const vs_batch* b) {
     return small ? kSmallShape : kDefaultShape;
 }
 
+// The step kernels' default.
+int step_shape(const vs_batch* b) {
+    int64_t cells = 0;
+    for (const TubeGrid& g : b->grids) cells += g.dims.interior_cells;
+    const int two = two_step_shape(cells);
+    if (tile_shape(two).kind == SHAPE_QUAD2 && shape_fits(b, two)) return two;
+    return single_step_shape(b);
+}
+
 int default_shape(const vs_batch* b) {
     // the resident kernel wherever the tubes fit it: it is the fastest from one
     // tube to 256 (us per step against the two-step strips: 5 tubes 0.74 / 2.7,
     // 96 tubes 4.0 / 7.6, 256 tubes 8.4 / 17.4); a single tube that does not
     // fit still keeps its state on one cluster
     if (shape_fits(b, cluster_shape()) && (!b->resident.order.empty() || b->grids.size() == 1)) return cluster_shape();
-    int64_t cells = 0;
-    for (const TubeGrid& g : b->grids) cells += g.dims.interior_cells;
-    const int two = two_step_shape(cells);
-    if (tile_shape(two).kind == SHAPE_QUAD2 && shape_fits(b, two)) return two;
-    return single_step_shape(b);
+    return step_shape(b);
+}
+
+// The shape of a run of `steps` steps.  A launch of the resident kernel reads
+// the maps and builds its tables before the first step, which costs more than
+// a few steps on the step kernels where the tubes fill the GPU.  Measured, us
+// per call past the wave front, resident / step kernels: 256 tubes 1 step 143 /
+// 55, 4 steps 150 / 101, 6 steps 167 / 166; 48 tubes 1 step 63 / 42, 4 steps 65 /
+// 52, 6 steps 69 / 73; 12 tubes 1 step 44 / 36, 2 steps 44 / 41, 3 steps 43 / 46.
+// Reference arithmetic: 256 tubes 4 steps 222 / 162, 6 steps 257 / 262.
+int run_shape(const vs_batch* b, int64_t steps) {
+    if (!b->default_run || b->resident.order.empty() || tile_shape(b->shape).kind != SHAPE_CLUSTER) return b->shape;
+    const size_t n = b->grids.size();
+    const int64_t few = n >= 40 ? 4 : n > 8 ? 1 : 0;
+    return steps <= few ? step_shape(b) : b->shape;
 }
 
 // Tile list of a launch shape, uploaded to a new device buffer (*n tiles).
@@ -1035,6 +1055,12 @@ int32_t run_status(const vs_batch* b) {
 void run_batch(vs_batch* b, int64_t steps, float* traces, int on_device) {
     const int n = (int)b->grids.size();
     if (b->shape < 0) b->shape = default_shape(b);
+    struct Restore {
+        vs_batch* b;
+        int shape;
+        ~Restore() { b->shape = shape; }
+    } restore{b, b->shape};
+    b->shape = run_shape(b, steps);
     build_tiles(b, b->shape);
     upload_sources(b, b->step + steps);
     const int64_t need = (int64_t)n * steps;
@@ -1780,6 +1806,7 @@ int vs_batch_set_tile(vs_batch* b, int32_t tile_index) {
     const int s = tile_index < 0 ? default_shape(b) : tile_index;
     if (!shape_fits(b, s)) return set_error(VS_ERR_UNSUPPORTED, "launch shape unavailable for this batch (shared memory, wall oscillator or fast_math)");
     b->shape = s;
+    b->default_run = tile_index < 0;
     return VS_OK;
 }
 
@@ -1819,6 +1846,7 @@ int vs_batch_autotune(vs_batch* b, int64_t steps, int32_t* best_index, float* be
         ck(cudaEventCreate(&e1), "event");
         float best = 1e30f;
         int best_i = default_shape(b);
+        b->default_run = false;
         for (int s = 0; s < tile_shape_count(); ++s) {
             if (!shape_fits(b, s)) continue;
             b->shape = s;
