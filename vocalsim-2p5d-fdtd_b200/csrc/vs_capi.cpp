@@ -21,6 +21,7 @@
 #include <memory>
 #include <new>
 #include <string>
+#include <system_error>
 #include <map>
 #include <vector>
 
@@ -57,8 +58,9 @@ constexpr size_t kGuard = 1024;  // bytes of slack around the tube planes of an 
 size_t align_up(size_t v) { return (v + kAlign - 1) / kAlign * kAlign; }
 
 // fn(i) for i in [0, n) on up to hardware_concurrency host threads (host
-// work only: map building, source tables, staging images); the first
-// exception thrown by a call is rethrown here after every thread joined.
+// work only: map building, source tables, staging images), the caller's among
+// them, and on fewer where the system gives no more; the first exception
+// thrown by a call is rethrown here after every thread joined.
 void parallel_for(size_t n, const std::function<void(size_t)>& fn) {
     size_t nt = std::min<size_t>(n, std::max(1u, std::thread::hardware_concurrency()));
     nt = std::min<size_t>(nt, 64);
@@ -69,19 +71,23 @@ void parallel_for(size_t n, const std::function<void(size_t)>& fn) {
     std::atomic<size_t> next{0};
     std::exception_ptr err;
     std::mutex m;
-    std::vector<std::thread> pool;
-    pool.reserve(nt);
-    for (size_t t = 0; t < nt; ++t)
-        pool.emplace_back([&] {
-            for (size_t i = next.fetch_add(1); i < n; i = next.fetch_add(1)) {
-                try {
-                    fn(i);
-                } catch (...) {
-                    std::lock_guard<std::mutex> lock(m);
-                    if (!err) err = std::current_exception();
-                }
+    auto work = [&] {
+        for (size_t i = next.fetch_add(1); i < n; i = next.fetch_add(1)) {
+            try {
+                fn(i);
+            } catch (...) {
+                std::lock_guard<std::mutex> lock(m);
+                if (!err) err = std::current_exception();
             }
-        });
+        }
+    };
+    std::vector<std::thread> pool;
+    pool.reserve(nt - 1);
+    try {
+        while (pool.size() + 1 < nt) pool.emplace_back(work);
+    } catch (const std::system_error&) {
+    }
+    work();
     for (std::thread& t : pool) t.join();
     if (err) std::rethrow_exception(err);
 }
@@ -1716,6 +1722,8 @@ int guarded(F&& f) {
         return set_error(VS_ERR_CUDA, std::string(e.where) + ": " + cudaGetErrorString(e.err));
     } catch (const std::bad_alloc&) {
         return set_error(VS_ERR_ALLOC, "host allocation failed");
+    } catch (const std::exception& e) {
+        return set_error(VS_ERR_ALLOC, std::string("host: ") + e.what());
     }
 }
 
