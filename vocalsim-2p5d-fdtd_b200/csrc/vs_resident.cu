@@ -32,7 +32,7 @@ void cluster_launch(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr, const Re
 
 bool resident_plan(const TubeGrid* grids, int n, int npairs, bool fast, ResidentPlan* out) {
     *out = ResidentPlan{};
-    if (npairs < 1 || npairs > kMaxPairs) return false;
+    if (npairs < 1 || npairs > kMaxPairs || n > 65535) return false;      // a tube per row of the grid
     int dev = 0, optin = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
