@@ -24,3 +24,14 @@ def test_nan_reaches_every_later_sample_and_no_earlier_one(cuda_ok):
     x[9000] = np.nan
     got = VA.audio(x, 2).cpu().numpy().ravel()
     assert np.all(np.isfinite(got[:4500])) and np.all(np.isnan(got[4500:]))
+
+
+@pytest.mark.parametrize("mul", [30, 64])
+@pytest.mark.parametrize("n", [17, 8193, 24600])
+def test_large_decimations(n, mul, cuda_ok):
+    """The scan's own error grows with srate_mul, to 4e-12 at 64: still the float32 rounding's tolerance."""
+    rng = np.random.default_rng(n + mul)
+    x = rng.standard_normal((2, n)).astype(np.float32)
+    got = VA.audio(x, mul).cpu().numpy()
+    for i in range(2):
+        assert np.max(np.abs(got[i] - OA.audio(x[i], mul))) <= 2.0 ** -22
