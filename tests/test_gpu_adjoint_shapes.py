@@ -4,21 +4,13 @@ import numpy as np
 import pytest
 
 import vocalsim_b200 as V
+from kernel_names import launched
 from vocalsim_b200 import synthetic as S
 
 pytestmark = pytest.mark.gpu
 SHAPES = range(len(V.tile_shapes()))
 CLUSTER = SHAPES[-1]
 TWO_STEP = next(k for k in SHAPES if V.tile_shape_steps(k) == 2)
-
-
-def kernels(call):
-    """Names of the kernels that `call` launches."""
-    import torch
-    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
-        call()
-        torch.cuda.synchronize()
-    return {e.name for e in prof.events()}
 
 
 def test_recomputation_follows_the_shape(cuda_ok):
@@ -31,11 +23,11 @@ def test_recomputation_follows_the_shape(cuda_ok):
                                (TWO_STEP, 48, "quad2"), (TWO_STEP, 63, None), (CLUSTER, 50, "resident_kernel")):
         b.set_tile(shape)
         b.forward_ckpt(steps, every)
-        names = kernels(lambda: out.append(b.adjoint(seed)))
-        history = {k for k in names if "adjoint" not in k and any(s in k for s in ("resident_", "quad", "strip_"))}
-        if part:
-            assert history and all(part in k for k in history), names
-        maps, gz = out.pop()
+        names = launched(lambda: out.append(b.adjoint(seed)), ("resident_kernel", "quad", "::strip_kernel"))
+        if part and names:
+            history = {k for k in names if "adjoint" not in k and any(s in k for s in ("resident_", "quad", "strip_"))}
+            assert all(part in k for k in history), names
+        maps, gz = out[-1]
         got = [gz] + [g for m in maps for g in m]
         want = want or got
         for x, y in zip(got, want):

@@ -1,11 +1,12 @@
 """The shared-memory cluster kernel (vs_cluster.cu) on the frames it is left with: those the resident kernel's plan
 refuses, here by their width (more than 1025 columns, or 961 with the two-mass source).  Values against the step
-kernels and the FP32 oracle; the profiler says which kernel ran."""
+kernels and the FP32 oracle; the profiler and the shape's limits say which kernel ran."""
 import numpy as np
 import pytest
 
 import oracle as O
 import vocalsim_b200 as V
+from kernel_names import launched
 
 pytestmark = pytest.mark.gpu
 CLUSTER = len(V.tile_shapes()) - 1
@@ -23,17 +24,19 @@ CASES = {"one": ({}, LONG[:1]), "one_sine_mouth": (dict(source_type=0, mouth_rad
          "two_mass_f64": (dict(TWO_MASS, tmm_f64=1), LONG[:1]), "two_mass_edge": (TWO_MASS, [tube(72.5, 2.0)])}
 
 
+KERNELS = ("cluster_kernel", "resident_kernel", "quad", "strip_kernel")
+
+
 def run(case, fast, shape, runs=(1, 130, 169)):
-    import torch
     kw, tubes = CASES[case]
     b = V.Batch([V.params(fast_math=fast, **kw) for _ in tubes], [V.Geometry(*t) for t in tubes])
     b.set_tile(shape)
-    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
-        trace = np.concatenate([b.run(n) for n in runs], axis=1)
+    trace = np.concatenate([b.run(n) for n in runs], axis=1)
     fields = [f for i in range(len(tubes)) for f in b.fields(i)]
+    names = launched(lambda: b.run(20), KERNELS)
     width = [d["frame_w"] for d in b.dims]
     b.close()
-    return trace, fields, {e.name for e in prof.events()}, width
+    return trace, fields, names, width
 
 
 @pytest.mark.parametrize("fast", [0, 1])
@@ -41,9 +44,10 @@ def run(case, fast, shape, runs=(1, 130, 169)):
 def test_wide_frames_equal_the_step_kernels(case, fast, cuda_ok):
     trace, fields, names, width = run(case, fast, CLUSTER)
     assert min(width) > (961 if case == "two_mass_edge" else 1025)
-    assert any("cluster_kernel" in k for k in names) and not any("resident_kernel" in k for k in names)
+    if names:
+        assert any("cluster_kernel" in k for k in names) and not any("resident_kernel" in k for k in names)
     want, want_fields, names, _ = run(case, fast, 21 if fast else 7)
-    assert not any("cluster_kernel" in k for k in names)
+    assert not any("cluster_kernel" in k for k in names or ())
     np.testing.assert_array_equal(trace, want)
     for x, y in zip(fields, want_fields):
         np.testing.assert_array_equal(x, y)
@@ -55,11 +59,22 @@ def test_wide_frames_equal_the_step_kernels(case, fast, cuda_ok):
 
 def test_frames_in_reach_run_on_the_resident_kernel(cuda_ok):
     """The widest frames either source's plan takes, and the default of one wide tube."""
-    import torch
     for kw, length, kernel in (({}, 75.0, "resident_kernel"), (TWO_MASS, 70.0, "resident_kernel"), ({}, 80.0, "cluster_kernel")):
         s = V.Solver(V.params(**kw), V.Geometry(*tube(length, 2.0)))
-        with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
-            got = s.run(60)
-        assert any(kernel in e.name for e in prof.events()), (s.dims["frame_w"], kernel)
+        got = s.run(60)
+        names = launched(lambda: s.run(20), KERNELS)
+        assert not names or any(kernel in k for k in names), (s.dims["frame_w"], kernel)
         np.testing.assert_array_equal(got, O.run(O.params(**kw), O.Geometry(*tube(length, 2.0)), 60, "f32"))
         s.close()
+
+
+def test_the_plan_refuses_wide_frames(cuda_ok):
+    """Only the shared-memory kernel is limited to 64 tubes: a wide batch of 65 has no cluster shape."""
+    for length, taken in ((80.0, False), (20.0, True)):
+        b = V.Batch([V.params() for _ in range(65)], [V.Geometry(*tube(length, 2.0)) for _ in range(65)])
+        if taken:
+            b.set_tile(CLUSTER)
+        else:
+            with pytest.raises(V.VsError):
+                b.set_tile(CLUSTER)
+        b.close()
