@@ -38,6 +38,7 @@ sys.path.insert(0, str(REPO / "vocalsim-2p5d-fdtd_b200" / "python"))
 N_TUBES = 256
 SIM_STEPS = 33075                      # 50 ms at 44.1 kHz x 15
 BYTES_PER_CELL_UPDATE = 37             # P,Vx,Vy read+write (24) + dP,dX,dY (12) + code (1)
+OPS_PER_CELL_UPDATE = 18               # 8 for the pressure, 5 for each velocity
 METRIC = "Gcell-updates/s"
 PEAKS = REPO / "MEASURED_PEAKS.json"
 FALLBACK_HBM_GBS = 6650.0
@@ -103,13 +104,14 @@ def hbm_peak():
     return FALLBACK_HBM_GBS, "fallback"
 
 
-def profiled_kernel(cells: int, shape: int, fast: int) -> dict:
+def profiled_kernel(cells: int, shape: int, fast: int, steps: int) -> dict:
     """DRAM bytes (read + write) per step-kernel launch and the issue-active
     percentage from the committed ncu summary of the same kernel (launch shape
     and arithmetic) on this same workload (same interior cell count); None
-    where no summary matches."""
+    where no summary matches.  A summary of a whole-run kernel gives the bytes
+    of a launch without steps and those of a step."""
     out = {"traffic": None, "issue_active_pct": None}
-    for name in ("quad2_kernel_fast_batch256.json", "quad_kernel_fast_batch256.json", "quad2_kernel_exact_batch256.json",
+    for name in ("resident_kernel_fast_batch256.json", "resident_kernel_exact_batch256.json", "quad2_kernel_fast_batch256.json", "quad_kernel_fast_batch256.json", "quad2_kernel_exact_batch256.json",
                  "strip_kernel_batch256.json"):
         f = REPO / "profiles" / name
         if not f.exists():
@@ -121,7 +123,7 @@ def profiled_kernel(cells: int, shape: int, fast: int) -> dict:
         if str(shape) in by_shape:
             out["traffic"] = int(by_shape[str(shape)]["dram_bytes_per_launch"])
         elif int(d.get("shape", -1)) == int(shape):
-            out["traffic"] = int(d["dram_bytes_per_launch"])
+            out["traffic"] = int(d["dram_bytes_per_launch"] + d.get("dram_bytes_per_step", 0) * steps)
         else:
             continue
         if str(shape) in by_shape and "smsp_issue_active_pct" in by_shape[str(shape)]:
@@ -436,7 +438,7 @@ def run_b200(args, rank, world):
         ba.close()
         return None
     if args.profile_single:
-        # profiling workload of the cluster kernel: the uniform 17.5 x 3 cm tube,
+        # profiling workload of the resident kernel on one tube: the uniform 17.5 x 3 cm tube,
         # `profile_single` steps in one launch after a 256-step warm-up launch
         from vocalsim_b200 import synthetic as S
         s1 = V.Solver(V.params(mu3d=0.005, uniform_depth_m=0.02, fast_math=fast), V.Geometry(*S.uniform_tube()))
@@ -486,7 +488,8 @@ def run_b200(args, rank, world):
     # a two-step shape advances two time steps per launch and moves the state
     # planes once per launch: algorithmic bytes per launch = 37 B x cells
     # (the resident kernel runs all steps in one launch and moves the planes and
-    # maps once; a launch that advances the step counter follows it)
+    # maps once; a launch that advances the step counter follows it: its roofline
+    # is FP32 issue, 18 operations per cell-update, one per lane and cycle)
     per_launch = V.tile_shape_steps(tile)
     whole = per_launch == 0
     if whole:
@@ -500,7 +503,14 @@ def run_b200(args, rank, world):
                     else BYTES_PER_CELL_UPDATE * cells * per_launch)
     achieved_gbs = launch_bytes / (launch_ms / 1e3) / 1e9
     peak, peak_kind = hbm_peak()
-    prof = profiled_kernel(cells, tile, fast)
+    prof = profiled_kernel(cells, tile, fast, sim_steps)
+    clock_rec = clocks.summary()
+    bound, unit, achieved, bound_peak = "hbm", "GB/s", achieved_gbs, peak
+    if whole:
+        sm_mhz, sms = clock_rec.get("sm_mhz") or 1965.0, torch.cuda.get_device_properties(dev).multi_processor_count
+        bound, unit, peak_kind = "fp32 issue (on chip)", "Gop/s", f"128 lanes x {sms} SMs x {sm_mhz:.0f} MHz"
+        achieved = OPS_PER_CELL_UPDATE * cells * sim_steps / (ms_step / 1e3) / 1e9
+        bound_peak = 128 * sms * sm_mhz / 1e3
 
     # ---- e2e: public API with host buffers: build + upload maps, run, download traces
     e2e = None
@@ -553,7 +563,7 @@ def run_b200(args, rank, world):
         b.record(stream)
         torch.cuda.synchronize()
         sms = a.elapsed_time(b)
-        single = {"workload": "uniform tube 17.5 x 3 cm, 57x253 frame, 33075 steps (cluster kernel: one launch)",
+        single = {"workload": "uniform tube 17.5 x 3 cm, 57x253 frame, 33075 steps (resident kernel: one launch)",
                   "value": round(s.dims["interior_cells"] * SIM_STEPS / (sms / 1e3) / 1e9, 3),
                   "unit": "Gcell-updates/s", "ms": round(sms, 2)}
         s.close()
@@ -600,7 +610,7 @@ def run_b200(args, rank, world):
         torch.cuda.synchronize()
         ms2 = a.elapsed_time(b)
         vowel_1s = {"workload": "vowel tube (seed 0, 44 sections, 3:1 elliptical), two-mass source 800 Pa in double, "
-                               f"1 s simulated ({n2} steps), one cluster-kernel launch",
+                               f"1 s simulated ({n2} steps), one launch",
                    "interior_cells": s2.dims["interior_cells"],
                    "value": round(s2.dims["interior_cells"] * n2 / (ms2 / 1e3) / 1e9, 3), "unit": "Gcell-updates/s",
                    "ms": round(ms2, 2), "s_per_simulated_s": round(ms2 / 1e3, 4)}
@@ -640,31 +650,33 @@ def run_b200(args, rank, world):
                 "parallelism": (f"LPT tube sharding of one {args.tubes}-tube batch x{world} (no collective)"
                                 if args.strong else f"tube sharding x{world} (no collective)"),
                 "arithmetic": "reciprocal form (fast_math=1)" if fast else "reference rounding (fast_math=0)",
-                "l2": ("state + maps per GPU > 126 MB L2, read once per timed step; no flush" if whole else
-                       "state + maps per GPU > 126 MB L2 and 33075 launches per timed step; no flush")},
-        "roofline": {"bound": "on-chip latency" if whole else "hbm", "achieved": round(achieved_gbs, 1), "peak": peak, "unit": "GB/s",
-                     "frac": round(achieved_gbs / peak, 4), "traffic": prof["traffic"],
+                "l2": ("a timed step resets, reads and writes some 160 MB (state, maps, traces) > 126 MB L2, once; no flush"
+                       if whole else "state + maps per GPU > 126 MB L2 and 33075 launches per timed step; no flush")},
+        "roofline": {"bound": bound, "achieved": round(achieved, 1), "peak": round(bound_peak, 1), "unit": unit,
+                     "frac": round(achieved / bound_peak, 4), "traffic": prof["traffic"],
                      # DRAM bytes the launch really moves (ncu, same kernel and workload) per
                      # launch time: the two-step kernel moves the planes once per two steps
-                     "dram_frac": (round(prof["traffic"] / (launch_ms / 1e3) / 1e9 / peak, 4)
+                     "dram_frac": (round(prof["traffic"] / (launch_ms / 1e3) / 1e9 / peak, 6)
                                    if prof["traffic"] else None),
                      "issue_active_pct": prof["issue_active_pct"],
                      # the metric's own form: Gcell-updates/s per GPU against the one-step
                      # roofline (37 B per cell-update moved once per step at the peak)
                      "gcell_roofline": round(peak / BYTES_PER_CELL_UPDATE, 1),
                      "gcell_frac": round(value / world / (peak / BYTES_PER_CELL_UPDATE), 4),
-                     "note": (f"{launch_bytes} B per launch (planes and maps once, traces) / " if whole else
+                     "note": (f"{OPS_PER_CELL_UPDATE} FP32 operations per cell-update x {cells} cells x {per_launch} time steps in "
+                              f"one launch ({launch_bytes} B algorithmic) / " if whole else
                               f"{BYTES_PER_CELL_UPDATE} B algorithmic per cell-update x {cells} cells x {per_launch} "
                               f"time step(s) per launch / ") +
-                             f"mean launch time {launch_ms * 1e3:.2f} us; peak {peak_kind}; "
-                             f"dram_frac and issue_active_pct from the committed ncu summary of the same kernel"},
+                             f"mean launch time {launch_ms * 1e3:.2f} us; peak {peak_kind}" +
+                             ("; dram_frac and issue_active_pct from the committed ncu summary of the same kernel"
+                              if prof["traffic"] else "; no committed ncu summary of this kernel on this workload")},
         "gpu_launches": args.steps * launches_per_forward,
-        "clocks": clocks.summary(),
+        "clocks": clock_rec,
         "e2e": e2e,
         "cpu_baseline": cpu,
         "single_tube": single,
         "vowel_1s": vowel_1s,
-        # against the library's default single-tube path (the cluster kernel), and
+        # against the library's default single-tube path (the resident kernel), and
         # against the same step kernels the batch uses, run on the one tube
         "batched_vs_single": round(value / world / single["value"], 2) if single else None,
         "batched_vs_single_step_kernels": round(value / world / single["step_kernels_value"], 2) if single else None,
@@ -689,7 +701,7 @@ def main():
     ap.add_argument("--profile-adjoint", type=int, default=0,
                     help="run a 16-tube checkpointed forward + adjoint of this many steps, untimed, for ncu")
     ap.add_argument("--profile-single", type=int, default=0,
-                    help="run the uniform tube for this many steps on the cluster kernel, untimed, for ncu")
+                    help="run the uniform tube for this many steps on the resident kernel, untimed, for ncu")
     ap.add_argument("--tile", type=int, default=-1)
     ap.add_argument("--no-e2e", action="store_true")
     ap.add_argument("--no-single", action="store_true")

@@ -375,8 +375,9 @@ int step_shape(const vs_batch* b) {
 
 int default_shape(const vs_batch* b) {
     // the resident kernel wherever the tubes fit it: it is the fastest from one
-    // tube to 256 (us per step against the two-step strips: 5 tubes 0.74 / 2.7,
-    // 96 tubes 4.0 / 7.6, 256 tubes 8.4 / 17.4); a single tube that does not
+    // tube to 256 (us per step against the two-step strips: 5 tubes 0.75 / 2.6,
+    // 96 tubes 4.0 / 7.6, 256 tubes 8.4 / 17.4; reference arithmetic: 5 tubes 1.1 /
+    // 4.4, 48 tubes 4.4 / 12.8, 256 tubes 18 / 34); a single tube that does not
     // fit still keeps its state on one cluster
     if (shape_fits(b, cluster_shape()) && (!b->resident.order.empty() || b->grids.size() == 1)) return cluster_shape();
     return step_shape(b);

@@ -1,7 +1,8 @@
 // vs_cluster.cu -- one tube on one thread-block cluster, a whole run per launch,
 // the bands in shared memory: the cluster shape of tubes the resident kernel
-// (vs_resident.cuh) does not take (more than 128 distinct descriptor pairs, or
-// more cells than its registers hold).
+// (vs_resident.cuh) does not take: frames of more than 1025 columns (961 with the
+// two-mass source), more rows than its registers hold, or more than 128 distinct
+// descriptor pairs.
 //
 // A single tube is too small to fill the GPU with one launch per step: the
 // graph-replayed step kernels spend most of each step in launch and memory

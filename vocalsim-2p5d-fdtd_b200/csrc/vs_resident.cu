@@ -45,7 +45,7 @@ bool resident_plan(const TubeGrid* grids, int n, int npairs, bool fast, Resident
     // clusters of 3 to 6 CTAs and 0.8 larger ones).  Measured, us per step:
     // 256 vowel tubes with 2 CTAs 9.6 (8.4 longest first), 3 CTAs 10.6, 4 CTAs
     // 10.8 (two-step strips 17.4); one 55 x 253 tube with 16 CTAs 0.69, 8 CTAs
-    // 0.81, 2 CTAs 1.9 (one band per CTA in vs_cluster.cu 1.35).
+    // 0.81, 2 CTAs 1.9 (two-step strips 2.5).
     bool tmm = false;
     for (int i = 0; i < n; ++i) tmm = tmm || grids[i].tmm;
     const int warps = kMaxWarps - (tmm ? 1 : 0);     // a warp for the two-mass model

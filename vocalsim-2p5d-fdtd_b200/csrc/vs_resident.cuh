@@ -42,9 +42,10 @@
 // time step (two-step strips 17.4), about 65 instructions per 64-cell row and
 // step at 0.4 per scheduler and cycle, half of the shared-memory pipe, the rest
 // the latency of a warp's own chain and the two barriers.  One 55 x 253 tube
-// (16 CTAs, 1 or 2 rows a lane): 0.65 us per step, 1.5 in the reference
-// arithmetic (a band per CTA with cells in branches: 1.35 and 3.7); with the
-// double two-mass model 0.91 (1.70).  Measured and not kept: scalar instead of
+// (16 CTAs, 1 or 2 rows a lane): 0.67 us per step, 1.1 in the reference
+// arithmetic (two-step strips 2.5 and 4.2), about 0.5 of it the exchange and the
+// two barriers; with the double two-mass model 0.88, its own chain of double
+// operations.  Measured and not kept: scalar instead of
 // packed operations (82 instructions, the same time); 64 registers for twice
 // the warps (spills, 16 us per step of the 256 tubes); 168 registers with 12
 // warps, taller groups, or a cluster size per tube (10.2 to 11.5 us).
